@@ -333,6 +333,18 @@ static int init_impl(const db_params* p, const double* gy_in, void* stream, db_c
     s.lrow = lr;
   }
   if ((rc = dalloc(c, &s.tri, (size_t)4 * np))) { db_finalize(c); g_init_err = c->err; return rc; }
+  if ((rc = dalloc(c, &s.cnr, (size_t)np))) { db_finalize(c); g_init_err = c->err; return rc; }
+  {
+    double4* d = nullptr;
+    if ((rc = dalloc(c, &d, (size_t)np))) { db_finalize(c); g_init_err = c->err; return rc; }
+    s.ryf = d;
+    std::vector<double4> r(np, make_double4(0.0, 0.0, 0.0, 0.0));
+    for (int j = 1; j <= Nyp; ++j)
+      r[j] = make_double4(1.0 / c->dyf[j], j < Nyp ? 1.0 / (c->dy[j + 1] * c->dyf[j]) : 0.0, 1.0 / c->dy[j + 1], 0.0);
+    if (cudaMemcpy(d, r.data(), np * sizeof(double4), cudaMemcpyHostToDevice) != cudaSuccess) {
+      db_finalize(c); g_init_err = "db_init: table upload failed"; return DB_ERR_CUDA;
+    }
+  }
   if ((rc = dalloc(c, &s.sc, 1))) { db_finalize(c); g_init_err = c->err; return rc; }
   g.flags = &s.sc->flags;
   size_t ntab = 4 * (size_t)np + g.kxs + g.nkzp;
@@ -892,7 +904,7 @@ static cudaError_t substep(db_ctx* c, int rk /* 0-based */, bool les) {
     if ((e = cudaStreamWaitEvent(st, c->ev_join, 0))) return e;
     if ((e = launch_rhs_cn(g, c->ph, s, rk, st))) return e;
     mark(c, rk, 6);
-    n += 4;
+    n += 5;
     // CFL on the last substep from the new velocity before the projection
     // (solver.f90:1241-1244): u1..u3 to physical space for it
     if (cfl_step) {
@@ -1258,9 +1270,8 @@ static int ensemble_steps_batched(db_ensemble* e, int nsteps) {
     }
     e->g_cap = c0->g;
     e->groups_cap = G;
-    // step scalars twice; per substep tri_coef, the two inverse passes,
-    // products, the z-pass, rhs_cn, cn_back and rem_div
-    e->bkernels = (long long)G * (2 + 3 * 8);
+    // step scalars twice and the substeps of every group
+    e->bkernels = (long long)G * (2 + 3 * substep_batch_kernels(c0->g));
   }
   for (int it = 0; it < nsteps; ++it) {
     if (cudaGraphLaunch(e->bgraph, e->st) != cudaSuccess) {

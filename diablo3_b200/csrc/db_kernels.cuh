@@ -22,13 +22,13 @@ constexpr int KT = 4;           // kx columns per z-pass CTA (kxs is a multiple 
 #ifndef DB_LB_FFT
 #define DB_LB_FFT 3
 #endif
+#ifndef DB_LB_ZPASS
+#define DB_LB_ZPASS 2
+#endif
 // k_rhs_cn: minimum resident 32-thread CTAs per SM (13 keeps every mode's
 // thread of a 512x512 plane resident at once: 128 registers)
 #ifndef DB_RHSCN_LB
 #define DB_RHSCN_LB 13
-#endif
-#ifndef DB_LB_ZPASS
-#define DB_LB_ZPASS 2
 #endif
 #ifndef DB_ZPASS_LAZY
 #define DB_ZPASS_LAZY 1
@@ -82,6 +82,18 @@ struct TriRow {
   double ef_lo, ef_hi;
   int is_bc, interior;
 };
+// What k_cn_solve needs of row j of the four equations, in z-pass order (0 u1,
+// 1 u3, 2 u2, 3 th): 1/b', u/b'; the answers of the row's chunk to unit
+// inflows from below and above; cn_hi, cn_lo; a' and its product from the
+// chunk's first row; the buoyancy weights of th_j, th_{j-1} and h / dy_j of
+// the u2 row; BC rows.  An odd number of 16-byte units (19), so that the rows
+// of a warp's chunks start in different banks.
+struct __align__(16) CnRow {
+  double ib[4][2], ab[4][2], cn[4][2];
+  double ap[4], qq[4];
+  double g[4];
+  int bc[4];
+};
 
 // Per-row constants of the AMD model (k_les_amd), host-computed once:
 // reciprocals of the spacings, the filter coefficients -2 C^2 Delta^2 at GY
@@ -128,6 +140,8 @@ struct State {
   double2* crs[4];                           // cr of u1, u3, u2, th (spectral FP64) for the spectral CN solve (no LES)
   double2* pfac;                             // rem_div factors: a' then 1/b', each np x sp doubles
   TriRow* tri;                               // 4 equations x np rows (th, u2, u1, u3)
+  CnRow* cnr;                                // np rows (k_tri_lu)
+  const double4* ryf;                        // np rows: 1/dyf_j, 1/(dy_{j+1} dyf_j) (0 on row Nyp), 1/dy_{j+1}
   DevScalars* sc;
   // LES (les_model_type 5), physical [j][z][x]; null without use_les
   double* gx[4];                             // d/dx of u1, u2, u3, th
@@ -195,6 +209,8 @@ MemberArgs member_args(const Geom& g, const Phys& ph, const State& s);
 // through the two events before the solves
 cudaError_t launch_substep_batch(const Geom& g, const Batch& b, int rk, cudaStream_t st, cudaStream_t st_side,
                                  cudaEvent_t ev_fork, cudaEvent_t ev_join);
+// the kernels launch_substep_batch launches
+int substep_batch_kernels(const Geom& g);
 // time_step += 1 (end = 0) or time += delta_t (end = 1) of every member
 cudaError_t launch_steps_batch(const Batch& b, int end, cudaStream_t st);
 // batched transforms (k_fft.cu): nf fields of every member from slot fin
@@ -213,7 +229,7 @@ cudaError_t launch_zpass_rhs(const Geom& g, const Phys& ph, const State& s, int 
 cudaError_t launch_tri_coef(const Geom& g, const Phys& ph, const State& s, int rk, cudaStream_t st);
 // the substep without LES: the nonlinear terms NL_e of the 4 equations into
 // spectral scratch (s.crs), then the spectral RHS joined with the CN solves
-// in spectral space (k_rhs_cn, k_cn_back), the state in place
+// in spectral space (k_rhs_cn, k_cn_back or k_cn_solve), the state in place
 cudaError_t launch_zpass_spec(const Geom& g, const State& s, cudaStream_t st);
 cudaError_t launch_rhs_cn(const Geom& g, const Phys& ph, const State& s, int rk, cudaStream_t st);
 

@@ -12,14 +12,14 @@
 //                  35-111) and the RK combination cr = cu + zeta h cf_old -
 //                  h grad p + beta h cf (solver.f90:396-456, 824-838,
 //                  966-973), cr through the inverse z-FFT to the physical solve.
-//  k_tri_coef    : the four implicit systems' rows incl. BC rows
-//                  (solver.f90:1012-1233, 1901-2324), LU-factored once per
+//  k_tri_rows,   : the four implicit systems' rows incl. BC rows
+//  k_tri_lu        (solver.f90:1012-1233, 1901-2324), LU-factored once per
 //                  substep (all (x,z) columns share them without LES).
 //  k_rhs_cn,     : without LES, after the forward z-FFT of the 8 fields: the
-//  k_cn_back       spectral RHS and the CN solves of th, u2, u1, u3 per
-//                  retained Fourier mode (explicit CN term + Thomas sweeps,
+//  k_cn_back, or   spectral RHS and the CN solves of th, u2, u1, u3 per
+//  k_cn_solve      retained Fourier mode (explicit CN term + Thomas sweeps,
 //                  solver.f90:850-870, 981-989, 1691-1852), FP64.
-//  k_rem_div     : per (kx,kz) column, divergence, complex Thomas, projection
+//  k_rem_div(_ch): per (kx,kz) column, divergence, complex Thomas, projection
 //                  and pressure update (solver.f90:1302-1379, 1261-1267).
 //  k_courant     : CFL reduction and dt scheduling (flow.f90:746-857).
 // The CN solves with eddy viscosity (one matrix per column) are in k_les.cu.
@@ -387,6 +387,7 @@ struct RhsIn {
   double2 nb2, nbp;     // e 0/1: cu2 of planes j and j+1; e 2: cth and cp of plane j-1
   double2 cfo;          // cf of the previous substep (rk > 0)
 };
+
 // a hint that brings the line holding p into L2 (p must be a valid global
 // address)
 __device__ __forceinline__ void prefetch_l2(const void* p) {
@@ -654,21 +655,20 @@ __global__ void __launch_bounds__(256) k_rhs_modes(const __grid_constant__ State
 }
 
 // ---------------------------------------------------------------------------
-// implicit systems: rows of the four equations (th, u2, u1, u3) -> tri[eq*np + j].
-// One CTA per equation: rows are filled in parallel in shared memory, the BC
-// rows and the forward elimination (a serial recurrence) by one thread.
+// implicit systems: rows of the four equations (th, u2, u1, u3) -> tri[eq*np + j],
+// one CTA per equation.  k_tri_rows fills the rows, every row by its own
+// thread, and sets the BC rows; k_tri_lu eliminates.
 // B: member-batched (blockIdx.y = member)
 template <bool B = false>
-__global__ void __launch_bounds__(256) k_tri_coef(Geom g0, Phys ph0, TriRow* tri0, DevScalars* sc0, int rk,
+__global__ void __launch_bounds__(256) k_tri_rows(Geom g0, Phys ph0, TriRow* tri0, CnRow* cnr0, DevScalars* sc0, int rk,
                                                   const MemberArgs* __restrict__ tab) {
   const int mb = B ? (int)blockIdx.y : 0;
   const Geom& g = g0;   // the same geometry for every member
   const Phys& ph = B ? tab[mb].ph : ph0;
-  TriRow* tri = B ? tab[mb].s.tri : tri0;
   DevScalars* sc = B ? tab[mb].s.sc : sc0;
-  extern __shared__ TriRow Rs[];
   const int eq = blockIdx.x;  // 0..3
   const int np = g.np, Nyp = g.ny;
+  TriRow* Rs = (B ? tab[mb].s.tri : tri0) + eq * np;
   const double temp1 = 0.5 * ph.nu * sc->h_bar[rk];
   const double tv = temp1 * ph.nu_v_scale;
   const double tth = temp1 / ph.pr * ph.nu_v_scale;
@@ -698,6 +698,10 @@ __global__ void __launch_bounds__(256) k_tri_coef(Geom g0, Phys ph0, TriRow* tri
         r.cn_lo = tv / dy[j] / dyf[j - 1];
         r.ef_lo = 0.5 / (dyf[j - 1] * dy[j]);   // times nu(j) + nu(j-1)
         r.ef_hi = 0.5 / (dyf[j] * dy[j]);       // times nu(j) + nu(j+1)
+        CnRow& q = (B ? tab[mb].s.cnr : cnr0)[j];
+        q.g[0] = ph.grav_y / (2.0 * dy[j]) * dyf[j - 1];
+        q.g[1] = ph.grav_y / (2.0 * dy[j]) * dyf[j];
+        q.g[2] = sc->h_bar[rk] / dy[j];
       } else {        // solver.f90:1140-1143, 1196-1199
         r.l = -tv / (dy[j] * dyf[j]);
         r.d = 1. - tv * (-1. / (dy[j + 1] * dyf[j]) - 1. / (dy[j] * dyf[j]));
@@ -757,24 +761,56 @@ __global__ void __launch_bounds__(256) k_tri_coef(Geom g0, Phys ph0, TriRow* tri
         setr(Nyp + 1, -1., 1., 0., dyf[Nyp] * ph.bc_c1[BC_V_MAX]);
       }
     }
-    // Thomas forward elimination of the matrix (thomas_forward_real_mpi with
-    // one rank: rows 1..Nyp+1, solver.f90:1731-1757)
-    double bprev = Rs[0].d;
-    Rs[0].ap = 0.0;
-    Rs[0].ibp = 1.0 / bprev;
-    double uprev = Rs[0].u;
+  }
+}
+
+// Thomas forward elimination of the matrix (thomas_forward_real_mpi with one
+// rank: rows 1..Nyp+1, solver.f90:1731-1757).  Only the pivots
+// b'_j = d_j - l_j u_{j-1} / b'_{j-1} form a chain: one thread runs it from
+// shared memory with one division per row, then a'_j = -l_j / b'_{j-1} and
+// 1 / b'_j follow with a thread per row, and what k_cn_solve's chunks need of
+// them: u_j / b'_j, the products of a' from the chunk's first row, and the
+// chunk's answers al_j, be_j to unit inflows from below and above.
+template <bool B = false>
+__global__ void __launch_bounds__(256) k_tri_lu(int np, int ch, TriRow* tri0, CnRow* cnr0, const MemberArgs* __restrict__ tab) {
+  const int eq = blockIdx.x, e = eq == 0 ? 3 : (eq == 1 ? 2 : eq - 2);   // k_tri_rows order -> z-pass order
+  TriRow* R = (B ? tab[blockIdx.y].s.tri : tri0) + eq * np;
+  CnRow* Q = B ? tab[blockIdx.y].s.cnr : cnr0;
+  extern __shared__ double2 ldu[];   // (d_j, l_j u_{j-1}), .x becomes b'_j; then (a'_j, 1/b'_j)
+  for (int j = threadIdx.x; j < np; j += blockDim.x)
+    ldu[j] = make_double2(R[j].d, j > 0 ? R[j].l * R[j - 1].u : 0.0);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double b = ldu[0].x;
     for (int j = 1; j < np; ++j) {
-      const double a = -Rs[j].l / bprev;
-      const double b = Rs[j].d + a * uprev;
-      Rs[j].ap = a;
-      Rs[j].ibp = 1.0 / b;
-      bprev = b;
-      uprev = Rs[j].u;
+      const double2 q = ldu[j];
+      b = q.x - q.y / b;
+      ldu[j].x = b;
     }
   }
   __syncthreads();
-  TriRow* R = tri + eq * np;
-  for (int j = threadIdx.x; j < np; j += blockDim.x) R[j] = Rs[j];
+  for (int j = threadIdx.x; j < np; j += blockDim.x) {
+    const double ap = j > 0 ? -R[j].l / ldu[j - 1].x : 0.0, ib = 1.0 / ldu[j].x;
+    R[j].ap = ap;
+    R[j].ibp = ib;
+    Q[j].ap[e] = ap;
+    Q[j].ib[e][0] = ib;
+    Q[j].ib[e][1] = R[j].u * ib;
+    Q[j].cn[e][0] = R[j].cn_hi;
+    Q[j].cn[e][1] = R[j].cn_lo;
+    Q[j].bc[e] = R[j].is_bc;
+  }
+  __syncthreads();
+  const int L = (np + ch - 1) / ch, j0 = threadIdx.x * L, j1 = min(np, j0 + L);   // the ch chunks of k_cn_solve
+  if (threadIdx.x < ch && j0 < j1) {
+    double q = 1.0, al = 0.0, be = 1.0;
+    for (int j = j0; j < j1; ++j) Q[j].qq[e] = (q *= Q[j].ap[e]);
+    for (int j = j1 - 1; j >= j0; --j) {
+      const double ib = Q[j].ib[e][0], uib = Q[j].ib[e][1];
+      Q[j].ab[e][0] = al = Q[j].qq[e] * ib - uib * al;
+      Q[j].ab[e][1] = be = -uib * be;
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -789,7 +825,10 @@ __global__ void __launch_bounds__(256) k_tri_coef(Geom g0, Phys ph0, TriRow* tri
 // solve and the forward transforms of the new state drop out, and the
 // solve runs in FP64 on both work types.  Real and imaginary parts of a
 // mode are two real columns of the same real system, with the LU factors
-// k_tri_coef shares.
+// k_tri_lu leaves.
+//
+// Two forms (cn_form): k_rhs_cn and k_cn_back walk all planes with one thread
+// per mode (many modes), k_cn_solve splits the planes into chunks.
 //
 // k_rhs_cn: one thread per retained mode walks the planes upward and runs
 // the four equations (z-pass order 0 u1, 1 u3, 2 u2, 3 th) together,
@@ -821,7 +860,7 @@ __global__ void __launch_bounds__(32, DB_RHSCN_LB) k_rhs_cn(const __grid_constan
   const int kzp = m / g.kxs, kx = m % g.kxs;
   const RhsK kc = rhs_consts(s, g, ph, rk, kx, kzp);
   const bool m0 = (m == 0);   // the (0,0) mode carries the BC constants
-  // z-pass order 0 u1, 1 u3, 2 u2, 3 th; k_tri_coef order th, u2, u1, u3
+  // z-pass order 0 u1, 1 u3, 2 u2, 3 th; k_tri_rows order th, u2, u1, u3
   const double2* const U[4] = {s.cu1 + m, s.cu3 + m, s.cu2 + m, s.cth + m};
   const int lo[4] = {g.jstart, g.jstart, 2, g.jstart_th};
   const int hi[4] = {g.jend, g.jend, g.ny, g.jend_th};
@@ -908,7 +947,7 @@ __global__ void __launch_bounds__(32, DB_RHSCN_LB) k_rhs_cn(const __grid_constan
 }
 
 // k_cn_back: back substitution per real column (2 sp doubles per plane)
-// and equation (blockIdx.y, k_tri_coef order th, u2, u1, u3) from the y
+// and equation (blockIdx.y, k_tri_rows order th, u2, u1, u3) from the y
 // values k_rhs_cn left in the scratch, batches of TB planes loaded first;
 // the new state is written on the planes the reference's solve stores,
 // the others keep their values.  A non-finite new state is reported as
@@ -956,6 +995,251 @@ __global__ void __launch_bounds__(128) k_cn_back(const __grid_constant__ State s
   }
   if (bad) atomicOr(B ? tab[mb].g.flags : g.flags, DB_FLAG_NONFINITE);
 }
+
+// k_cn_solve: a CTA owns M neighbouring modes over all planes and runs the
+// four equations (z-pass order 0 u1, 1 u3, 2 u2, 3 th) together.  The planes
+// are split into CHN chunks of L rows, one thread per (chunk, mode), because
+// one thread per mode walking every plane is bound by the latency of its
+// own chain of loads (3.5 us per plane, whatever the size of the grid).
+//  1  RHS, forward sweep and back substitution within the chunk, from zero
+//     inflow at both of its ends: NL from the z-pass (or its Z(N), Z(M)
+//     parts, SPLITZ), cf (stored) and cr (solver.f90:396-609, 824-838,
+//     966-973, 35-111), the explicit CN term from the old state planes
+//     j-1..j+1, y_j = v_j + a'_j y_{j-1}, x_j = y_j/b'_j - (u_j/b'_j) x_{j+1};
+//  2  the inflows of every chunk: y from below, y_out(c) = y_local(c) + P_c
+//     y_out(c-1), then x from above, x_out(c) = x_local(c) + al y_in(c) +
+//     be x_out(c+1), each a warp scan over the chunks;
+//  3  x_j = x_local_j + al_j y_in + be_j x_in, the new state written on the
+//     planes the reference's solve stores (the others keep their values).
+// al_j, be_j are the chunk's answers to unit inflows, the same for every mode
+// (k_tri_lu).  Every state, history and NL plane crosses HBM once and y, x
+// never do (a forward and a back-substitution kernel would write and read
+// them).  The rows are diagonally dominant, so the split adds rounding of
+// the same size as the sweeps' own.  A non-finite new state is reported as
+// DB_FLAG_NONFINITE.  B: member-batched (blockIdx.y = member)
+// The rows' constants (CnRow, laid out by k_tri_lu) are copied to shared
+// memory: read from global memory they missed L1 behind the planes' stream,
+// and that latency, in every step of every sweep, bounded the kernel.
+template <int M, int CHN>
+constexpr size_t cn_smem(int np) {
+  return ((size_t)np * 4 * M + (size_t)4 * M * (CHN + 1)) * sizeof(double2) + (size_t)np * sizeof(CnRow);
+}
+
+// inclusive scan y_c <- y_c + p_c y_{c-1} over lanes c of segments of CHN lanes
+template <int CHN>
+__device__ __forceinline__ double2 chunk_scan(double2 y, double p, int c) {
+#pragma unroll
+  for (int d = 1; d < CHN; d <<= 1) {
+    const double yx = __shfl_up_sync(0xffffffffu, y.x, d, CHN), yy = __shfl_up_sync(0xffffffffu, y.y, d, CHN);
+    const double po = __shfl_up_sync(0xffffffffu, p, d, CHN);
+    if (c >= d) {
+      y.x += p * yx;
+      y.y += p * yy;
+      p *= po;
+    }
+  }
+  return y;
+}
+// chunk c of a column in lane c: from its last y and first x (zero inflow) to
+// y_in from below and the final x of its first row, the chunk below's x_in
+template <int CHN>
+__device__ __forceinline__ void chunk_inflows(double2& y, double2& x, double p, double al, double be, int c) {
+  const double2 q = chunk_scan<CHN>(y, p, c);
+  y.x = __shfl_up_sync(0xffffffffu, q.x, 1, CHN);
+  y.y = __shfl_up_sync(0xffffffffu, q.y, 1, CHN);
+  if (c == 0) y = make_double2(0.0, 0.0);
+  x.x += al * y.x;
+  x.y += al * y.y;
+  const int rc = CHN - 1 - c;   // the same scan with the chunks in reverse
+  x.x = __shfl_sync(0xffffffffu, x.x, rc, CHN);
+  x.y = __shfl_sync(0xffffffffu, x.y, rc, CHN);
+  be = __shfl_sync(0xffffffffu, be, rc, CHN);
+  x = chunk_scan<CHN>(x, be, c);
+  x.x = __shfl_sync(0xffffffffu, x.x, rc, CHN);
+  x.y = __shfl_sync(0xffffffffu, x.y, rc, CHN);
+}
+
+// r + a v, r + i a v
+__device__ __forceinline__ double2 axpy(double2 r, double a, double2 v) {
+  return make_double2(r.x + a * v.x, r.y + a * v.y);
+}
+__device__ __forceinline__ double2 axpy_i(double2 r, double a, double2 v) {
+  return make_double2(r.x - a * v.y, r.y + a * v.x);
+}
+
+template <int M, int CHN, bool SPLITZ, bool B = false>
+__global__ void __launch_bounds__(CHN * M) k_cn_solve(const __grid_constant__ State s0, Geom g0, Phys ph0, int rk,
+                                                        const __grid_constant__ FieldSet nl0,
+                                                        const MemberArgs* __restrict__ tab) {
+  const int mb = B ? (int)blockIdx.y : 0;
+  const State& s = B ? tab[mb].s : s0;
+  const Geom& g = g0;   // the same geometry for every member
+  const Phys& ph = B ? tab[mb].ph : ph0;
+  const FieldSet& nl = B ? tab[mb].fs[FS_NL] : nl0;
+  extern __shared__ __align__(16) unsigned char sm_raw[];
+  const int np = g.np;
+  double2* ys = reinterpret_cast<double2*>(sm_raw);          // [np][4][M]: y, then x within the chunk
+  double2* yb = ys + (size_t)np * 4 * M;                     // last y of a chunk, then its y_in: [4][M][CHN + 1]
+  CnRow* rows = reinterpret_cast<CnRow*>(yb + 4 * M * (CHN + 1));   // [np]
+  {
+    const double2* src = reinterpret_cast<const double2*>(s.cnr);
+    double2* dst = reinterpret_cast<double2*>(rows);
+    const int n2 = np * (int)(sizeof(CnRow) / sizeof(double2));
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n2; i += CHN * M) dst[i] = src[i];
+  }
+  __syncthreads();
+  const int mi = threadIdx.x % M, c = threadIdx.x / M;
+  const long long sp = g.sp;
+  const long long m = (long long)blockIdx.x * M + mi;
+  const bool live = m < sp;
+  const int L = (np + CHN - 1) / CHN;
+  const int j0 = c * L, j1 = live ? min(np, j0 + L) : j0;   // rows j0 .. j1-1 (none past the last plane)
+  const double2 Z2 = make_double2(0.0, 0.0);
+  {
+    double2 y[4] = {Z2, Z2, Z2, Z2};
+    if (j0 < j1) {
+      double2 x[4] = {Z2, Z2, Z2, Z2};
+      const int kzp = (int)(m / g.kxs), kx = (int)(m % g.kxs);
+      const RhsK kc = rhs_consts(s, g, ph, rk, kx, kzp);
+      const bool m0 = (m == 0);   // the (0,0) mode carries the BC constants
+      const double f = ph.ro_inv / ph.delta;
+      const double tw = ph.front_tw ? ph.delta / ph.ro_inv : 0.0;   // thermal wind of the front
+      const double qt = tw * (ph.dthdx * kc.kzv - ph.dthdz * kc.kxv);
+      const double c1 = -(ph.dthdz * tw), c3 = ph.dthdx * tw;
+      const double nk = -ph.nu * kc.kk, nkt = -(ph.nu / ph.pr) * kc.kk;
+      const double gb = m0 ? 0.0 : 1.0;   // no buoyancy in the mean u2 equation
+      const double kxp = -kc.temp4 * kc.kxv, kzq = -kc.temp4 * kc.kzv;
+      double fx = 0.0;   // mean forcing of u1
+      if (m0 && ph.f_type == 1) fx = -kc.temp4 * ph.px0;
+      if (m0 && ph.f_type == 2) fx = -kc.temp4 * (ph.px0 + ph.amp_omega0 * cos(ph.omega0 * s.sc->time));
+      const bool old = rk > 0;
+      long long a = j0 * sp + m;
+      double2 um[4], uc[4];
+      const double2* const u1p = s.cu1; const double2* const u3p = s.cu3;
+      const double2* const u2p = s.cu2; const double2* const thp = s.cth;
+      um[0] = um[1] = um[2] = um[3] = Z2;
+      double2 pm = Z2;   // cp of plane j-1
+      if (j0 > 0) {
+        um[0] = u1p[a - sp]; um[1] = u3p[a - sp]; um[2] = u2p[a - sp]; um[3] = thp[a - sp];
+        pm = s.cp[a - sp];
+      }
+      uc[0] = u1p[a]; uc[1] = u3p[a]; uc[2] = u2p[a]; uc[3] = thp[a];
+      for (int j = j0; j < j1; ++j, a += sp) {
+        const bool rv = in_rng(j, g.jstart, g.jend), r2 = in_rng(j, 2, g.ny), rt = in_rng(j, g.jstart_th, g.jend_th);
+        double2 un[4] = {Z2, Z2, Z2, Z2}, n4[4] = {Z2, Z2, Z2, Z2}, z4[4] = {Z2, Z2, Z2, Z2}, h4[4] = {Z2, Z2, Z2, Z2};
+        if (j + 1 < np) { un[0] = u1p[a + sp]; un[1] = u3p[a + sp]; un[2] = u2p[a + sp]; un[3] = thp[a + sp]; }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const bool rr = e < 2 ? rv : (e == 2 ? r2 : rt);
+          if (rr) n4[e] = ((const double2*)nl.p[e])[a];
+          if (SPLITZ && rr) z4[e] = ((const double2*)nl.p[4 + e])[a];
+          if (rr && old) h4[e] = rhs_cf(s, e)[a];
+        }
+        const double2 cp = s.cp[a];
+        const CnRow& row = rows[j];
+        double sf = 0.0, sg = 0.0;
+        if (ph.front_tw) {
+          sf = (g.gyf[j] - 0.5 * ph.ly) * qt;
+          sg = (g.gy[j] - 0.5 * ph.ly) * qt;
+        }
+        const double2 v2 = make_double2(0.5 * (uc[2].x + un[2].x), 0.5 * (uc[2].y + un[2].y));
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const bool rr = e < 2 ? rv : (e == 2 ? r2 : rt);
+          const double2 u = uc[e];
+          const double2 n = n4[e], h = h4[e], z = z4[e];
+          double2 w;
+          {
+            double2 cf = make_double2(u.x * (e == 3 ? nkt : nk), u.y * (e == 3 ? nkt : nk));
+            cf = axpy_i(cf, -(e == 2 ? sg : sf), u);
+            if (e == 0) cf = axpy(axpy(axpy(cf, f, uc[1]), ph.grav_x, uc[3]), -c1, v2);
+            if (e == 1) cf = axpy(axpy(axpy(cf, -f, uc[0]), ph.grav_z, uc[3]), -c3, v2);
+            if (e == 2) cf = axpy(axpy(cf, gb * row.g[0], uc[3]), gb * row.g[1], um[3]);
+            if (e == 3) cf = axpy(axpy(cf, -ph.dthdx, uc[0]), -ph.dthdz, uc[1]);
+            cf.x -= n.x;
+            cf.y -= n.y;
+            if (SPLITZ) cf = axpy_i(cf, -kc.kzv, z);   // NL = Z(N) + i kz Z(M), both already scaled by 1/Nz
+            if (rr) rhs_cf(s, e)[a] = cf;
+            w = axpy(axpy(u, kc.temp5, cf), kc.temp3, h);
+            if (e == 0) {
+              w = axpy_i(w, kxp, cp);
+              w.x += fx;
+            }
+            if (e == 1) w = axpy_i(w, kzq, cp);
+            if (e == 2) w = axpy(w, -row.g[2], make_double2(cp.x - pm.x, cp.y - pm.y));
+          }
+          const double ch = row.cn[e][0], cl = row.cn[e][1];
+          w.x += ch * (un[e].x - u.x) - cl * (u.x - um[e].x);
+          w.y += ch * (un[e].y - u.y) - cl * (u.y - um[e].y);
+          if (row.bc[e]) w = make_double2(m0 ? s.tri[(e == 0 ? 2 : e == 1 ? 3 : e == 2 ? 1 : 0) * np + j].bc : 0.0, 0.0);
+          y[e] = axpy(w, row.ap[e], y[e]);   // a' = 0 on row 0
+          ys[(j * 4 + e) * M + mi] = y[e];
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          um[e] = uc[e];
+          uc[e] = un[e];
+        }
+        pm = cp;
+      }
+#pragma unroll 2
+      for (int j = j1 - 1; j >= j0; --j) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const double ib = rows[j].ib[e][0], uib = rows[j].ib[e][1];
+          double2* q = ys + (j * 4 + e) * M + mi;
+          x[e].x = q->x * ib - uib * x[e].x;
+          x[e].y = q->y * ib - uib * x[e].y;
+          *q = x[e];
+        }
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) yb[(e * M + mi) * (CHN + 1) + c] = y[e];
+  }
+  __syncthreads();
+  {   // 32 / CHN modes a warp, one lane per chunk; ys[f0] becomes the final x
+    const int lane = threadIdx.x & 31, cc = lane % CHN;
+    const int mm = (threadIdx.x >> 5) * (32 / CHN) + lane / CHN;
+    const int f0 = cc * L, f1 = min(np, f0 + L) - 1;
+    const bool on = f0 < np && (long long)blockIdx.x * M + mm < sp;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      double2* const q = yb + (e * M + mm) * (CHN + 1) + cc;
+      double2* const xq = ys + ((on ? f0 : 0) * 4 + e) * M + mm;
+      double2 y = on ? *q : Z2, x = on ? *xq : Z2;
+      chunk_inflows<CHN>(y, x, on ? rows[f1].qq[e] : 0.0, on ? rows[f0].ab[e][0] : 0.0, on ? rows[f0].ab[e][1] : 0.0, cc);
+      if (on) {
+        *q = y;
+        *xq = x;
+      }
+    }
+  }
+  __syncthreads();
+  bool bad = false;
+  double2 yin[4], xin[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    yin[e] = yb[(e * M + mi) * (CHN + 1) + c];
+    xin[e] = j1 > j0 && j1 < np ? ys[(j1 * 4 + e) * M + mi] : Z2;   // first row of the chunk above
+  }
+#pragma unroll 2
+  for (int j = j0; j < j1; ++j) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      double2 x = ys[(j * 4 + e) * M + mi];
+      if (j > j0) x = axpy(axpy(x, rows[j].ab[e][0], yin[e]), rows[j].ab[e][1], xin[e]);
+      bad = bad || !(fabs(x.x) <= 1.7976931348623157e308) || !(fabs(x.y) <= 1.7976931348623157e308);
+      const int slo = (e < 2 ? g.jstart : (e == 2 ? 2 : g.jstart_th)) - 1;
+      const int shi = (e < 2 ? g.jend : (e == 2 ? g.ny : g.jend_th)) + 1;
+      double2* u = e == 0 ? s.cu1 : (e == 1 ? s.cu3 : (e == 2 ? s.cu2 : s.cth));
+      if (j >= slo && j <= shi) u[j * sp + m] = x;
+    }
+  }
+  if (bad) atomicOr(B ? tab[mb].g.flags : g.flags, DB_FLAG_NONFINITE);
+}
+
 // ---------------------------------------------------------------------------
 // rem_div factors: per (kx, kzp) column, rows 1..Nyp of the Poisson system
 // (solver.f90:1326-1333 with apply_BC_rem_div_mpi 2341-2368), forward
@@ -1096,6 +1380,123 @@ __global__ void __launch_bounds__(128, LB) k_rem_div(const __grid_constant__ Sta
       if (update_cp && j >= g.jstart && j <= g.jend) cpp[a + q0] = pc[c] + phi * itemp4;
       phin = phi;
     }
+  }
+}
+
+// The same for fewer modes (go_rem_div), as k_cn_solve: a CTA owns M modes, the rows 1..Nyp of a column are split
+// into CHN chunks with one thread each, swept from zero inflow, and the
+// inflows come from warp scans over the chunks (one thread per column walking
+// all rows was bound by its chain of loads, 0.9 us per row on any grid).  The
+// Poisson matrix of a (kx, kzp) column is real, so one set of factors and
+// unit answers (al, be; kept beside phi) serves both parts of phi, and every
+// factor is read once.  B: member-batched (blockIdx.y = member).
+template <int M, int CHN>
+constexpr size_t rem_div_smem(int np) {
+  return (size_t)2 * np * M * sizeof(double2) + (size_t)M * (CHN + 1) * (sizeof(double2) + sizeof(double));
+}
+template <int M, int CHN, bool B = false>
+__global__ void __launch_bounds__(CHN * M, 3) k_rem_div_ch(const __grid_constant__ State s0, Geom g0, int rk, int update_cp,
+                                                        const MemberArgs* __restrict__ tab) {
+  const int mb = B ? (int)blockIdx.y : 0;
+  const State& s = B ? tab[mb].s : s0;
+  const Geom& g = g0;   // the same geometry for every member
+  extern __shared__ __align__(16) unsigned char sm_raw[];
+  const int Nyp = g.ny, np = g.np;
+  const long long sp = g.sp;
+  const int mi = threadIdx.x % M, c = threadIdx.x / M;
+  const long long m = (long long)blockIdx.x * M + mi;
+  const int kzp = (int)(m / g.kxs), kx = (int)(m % g.kxs);
+  const bool live = m < sp && kx <= g.nkx;
+  double2* gs = reinterpret_cast<double2*>(sm_raw);          // [np][M] g, then phi within the chunk
+  double2* ab = gs + (size_t)np * M;                         // [np][M] (prod a', -), then (al, be)
+  double2* yb = ab + (size_t)np * M;                         // [M][CHN + 1] last g of a chunk, then its inflow
+  double* pb = reinterpret_cast<double*>(yb + M * (CHN + 1));   // [M][CHN + 1] prod a' of a chunk
+  const int L = (Nyp + CHN - 1) / CHN;
+  const int j0 = 1 + c * L, j1 = live ? min(Nyp + 1, j0 + L) : j0;   // rows j0 .. j1-1
+  const double kxv = live ? g.kx[kx] : 0.0, kzv = live ? g.kz[kzp] : 0.0;
+  // forward sweep: g_1 = 0 (BC row), g_j = rhs_j + a'_j g_{j-1}; rhs_Nyp = 0
+  {
+    double2 y = make_double2(0.0, 0.0), x = make_double2(0.0, 0.0);
+    double pr = 1.0, al = 0.0, be = 1.0;
+    if (j0 < j1) {
+      const double2* u1 = s.cu1 + m;
+      const double2* u3 = s.cu3 + m;
+      const double2* u2 = s.cu2 + m;
+      const double* pfa = pfac_a(s, g) + m;
+      const double* pfb = pfac_ib(s, g) + m;
+      double2 u2c = u2[j0 * sp];
+#pragma unroll 3
+      for (int j = j0; j < j1; ++j) {
+        const double2 u2n = u2[(j + 1) * sp];
+        const double2 a1 = u1[j * sp], a3 = u3[j * sp];
+        const double pa = pfa[j * sp];   // 0 on row 1
+        const double idf = s.ryf[j].x;   // 1 / dyf on rows 2..Nyp-1
+        double2 rhs = make_double2((u2n.x - u2c.x) * idf, (u2n.y - u2c.y) * idf);
+        rhs = axpy_i(axpy_i(rhs, kxv, a1), kzv, a3);
+        if (j == 1 || j == Nyp) rhs = make_double2(0.0, 0.0);
+        y = axpy(rhs, pa, y);
+        pr *= pa;
+        gs[j * M + mi] = y;
+        ab[j * M + mi].x = pr;
+        u2c = u2n;
+      }
+      // phi_j = (g_j - cj phi_{j+1}) / b'_j
+#pragma unroll 3
+      for (int j = j1 - 1; j >= j0; --j) {
+        const double ib = pfb[j * sp];
+        double cj = s.ryf[j].y;
+        if (j == 1) cj = m == 0 ? 0.0 : -1.0;
+        const double ci = cj * ib;
+        double2* q = gs + j * M + mi;
+        double2* r = ab + j * M + mi;
+        x = make_double2(q->x * ib - ci * x.x, q->y * ib - ci * x.y);
+        al = r->x * ib - ci * al;
+        be *= -ci;
+        *q = x;
+        *r = make_double2(al, be);
+      }
+    }
+    yb[mi * (CHN + 1) + c] = y;
+    pb[mi * (CHN + 1) + c] = pr;
+  }
+  __syncthreads();
+  {   // 32 / CHN modes a warp, one lane per chunk; gs[f0] becomes the final phi
+    const int lane = threadIdx.x & 31, cc = lane % CHN;
+    const int mm = (threadIdx.x >> 5) * (32 / CHN) + lane / CHN;
+    const long long mg = (long long)blockIdx.x * M + mm;
+    const int f0 = 1 + cc * L;
+    const bool on = f0 <= Nyp && mg < sp && (int)(mg % g.kxs) <= g.nkx;
+    const int q = mm * (CHN + 1) + cc, r = (on ? f0 : 0) * M + mm;
+    double2 y = make_double2(0.0, 0.0), x = y, w = y;
+    if (on) {
+      y = yb[q];
+      x = gs[r];
+      w = ab[r];
+    }
+    chunk_inflows<CHN>(y, x, on ? pb[q] : 0.0, w.x, w.y, cc);
+    if (on) {
+      yb[q] = y;
+      gs[r] = x;
+    }
+  }
+  __syncthreads();
+  // phi with the projection (solver.f90:1361-1376) and cp update
+  const double itemp4 = 1.0 / s.sc->h_bar[rk];
+  const double2 yin = yb[mi * (CHN + 1) + c];
+  const double2 xin = j1 > j0 && j1 <= Nyp ? gs[j1 * M + mi] : make_double2(0.0, 0.0);   // first row of the chunk above
+  double2 phin = xin;   // phi of row j+1
+#pragma unroll 3
+  for (int j = j1 - 1; j >= j0; --j) {
+    const long long a = j * sp + m;
+    const double2 r = ab[j * M + mi];
+    double2 phi = gs[j * M + mi];
+    if (j > j0) phi = axpy(axpy(phi, r.x, yin), r.y, xin);
+    s.cu1[a] = axpy_i(s.cu1[a], -kxv, phi);
+    s.cu3[a] = axpy_i(s.cu3[a], -kzv, phi);
+    if (j + 1 <= Nyp)   // u2(j+1) -= Dy phi
+      s.cu2[a + sp] = axpy(s.cu2[a + sp], -s.ryf[j].z, make_double2(phin.x - phi.x, phin.y - phi.y));
+    if (update_cp && j >= g.jstart && j <= g.jend) s.cp[a] = axpy(s.cp[a], itemp4, phi);
+    phin = phi;
   }
 }
 
@@ -1328,7 +1729,7 @@ cudaError_t launch_zpass_rhs(const Geom& g, const Phys& ph, const State& s, int 
 // without LES: the nonlinear terms into spectral scratch, then the spectral
 // RHS with the CN solves.  FP64 fields: Z(N_e) / Nz into s.crs[e] and
 // Z(M_e) / Nz into s.nls[4 + e] (k_fwd_z, 4-column CTAs), combined in
-// k_rhs_cn; FP32 fields: NL_e into s.crs[e] (k_fwd_z_nl).
+// k_cn_solve; FP32 fields: NL_e into s.crs[e] (k_fwd_z_nl).
 cudaError_t launch_zpass_spec(const Geom& g, const State& s, cudaStream_t st) {
   if (!s.crs[0] || (!g.prec && !s.nls[4])) return cudaErrorInvalidValue;
   if (!g.prec)
@@ -1337,18 +1738,74 @@ cudaError_t launch_zpass_spec(const Geom& g, const State& s, cudaStream_t st) {
   return launch_fwd_z_nl(g, fset(s.xh[0], s.xh[1], s.xh[2], s.xh[3], s.xh[4], s.xh[5], s.xh[6], s.xh[7]),
                          fset(s.crs[0], s.crs[1], s.crs[2], s.crs[3]), st);
 }
+// Modes per CTA of k_cn_solve (0: k_rhs_cn and k_cn_back).  One thread per
+// mode needs tens of thousands of modes to hide its chain of loads; the chunked
+// form has 4 to 32 times the threads.  Two-kernel -> chunked, us a substep:
+// 64x65x64 261 -> 11, 256x129x256 666 -> 237, 512x129x256 756 -> 444, 32
+// channels of 128x65x128 (mixed) 947 -> 844, but 512x257x512 2050 -> 2200, so
+// planes of more than 36000 modes keep the two kernels.  Wide CTAs read longer
+// rows and scan less (32 channels: 1363 with 8 modes, 999 with 16, 844 with
+// 32), so the widest one whose columns fit shared memory and that still gives
+// two thirds of the SMs a CTA (64x65x64: 11 with 8 modes, 21 with 32).  It
+// depends on the channel only, so a member of an ensemble gives the bits of
+// its solo run.
+constexpr size_t SMEM_CTA = 227 * 1024;
+constexpr long long CH_MODES = 36000, CH_CTAS = 96;
+static int cn_form(const Geom& g) {
+  if (g.sp > CH_MODES) return 0;
+  if (cn_smem<32, 8>(g.np) <= SMEM_CTA && g.sp >= 32 * CH_CTAS) return 32;
+  if (cn_smem<16, 16>(g.np) <= SMEM_CTA && g.sp >= 16 * CH_CTAS) return 16;
+  if (cn_smem<8, 32>(g.np) <= SMEM_CTA) return 8;
+  if (cn_smem<4, 32>(g.np) <= SMEM_CTA) return 4;
+  return 0;
+}
+static int cn_chunks(const Geom& g) { return cn_form(g) == 32 ? 8 : (cn_form(g) == 16 ? 16 : 32); }
+template <int M, int CHN, bool SPLITZ, bool B>
+static cudaError_t go_cn_solve_t(const Geom& g, const Phys& ph, const State& s, int rk, const FieldSet& nl,
+                                 const MemberArgs* tab, int n, cudaStream_t st) {
+  const size_t smem = cn_smem<M, CHN>(g.np);
+  const cudaError_t e = cudaFuncSetAttribute(k_cn_solve<M, CHN, SPLITZ, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e) return e;
+  k_cn_solve<M, CHN, SPLITZ, B><<<dim3((unsigned)((g.sp + M - 1) / M), n), CHN * M, smem, st>>>(s, g, ph, rk, nl, tab);
+  return cudaGetLastError();
+}
+template <bool SPLITZ, bool B>
+static cudaError_t go_cn(const Geom& g, const Phys& ph, const State& s, int rk, const FieldSet& nl,
+                         const MemberArgs* tab, int n, cudaStream_t st) {
+  switch (cn_form(g)) {
+    case 32: return go_cn_solve_t<32, 8, SPLITZ, B>(g, ph, s, rk, nl, tab, n, st);
+    case 16: return go_cn_solve_t<16, 16, SPLITZ, B>(g, ph, s, rk, nl, tab, n, st);
+    case 8: return go_cn_solve_t<8, 32, SPLITZ, B>(g, ph, s, rk, nl, tab, n, st);
+    case 4: return go_cn_solve_t<4, 32, SPLITZ, B>(g, ph, s, rk, nl, tab, n, st);
+  }
+  k_rhs_cn<SPLITZ, B><<<dim3((unsigned)((g.sp + 31) / 32), n), 32, 0, st>>>(s, g, ph, rk, nl, tab);
+  k_cn_back<B><<<dim3((unsigned)((2 * g.sp + 127) / 128), 4, n), 128, 0, st>>>(s, g, nl, tab);
+  return cudaGetLastError();
+}
+template <bool B>
+static cudaError_t go_cn_solve(const Geom& g, const Phys& ph, const State& s, int rk, const FieldSet& nl,
+                               const MemberArgs* tab, int n, cudaStream_t st) {
+  return g.prec ? go_cn<false, B>(g, ph, s, rk, nl, tab, n, st) : go_cn<true, B>(g, ph, s, rk, nl, tab, n, st);
+}
+int substep_batch_kernels(const Geom& g) { return cn_form(g) ? 8 : 9; }
 cudaError_t launch_rhs_cn(const Geom& g, const Phys& ph, const State& s, int rk, cudaStream_t st) {
   const FieldSet nl = fset(s.crs[0], s.crs[1], s.crs[2], s.crs[3], s.nls[4], s.nls[5], s.nls[6], s.nls[7]);
-  if (!g.prec) k_rhs_cn<true><<<(unsigned)((g.sp + 31) / 32), 32, 0, st>>>(s, g, ph, rk, nl, nullptr);
-  else k_rhs_cn<false><<<(unsigned)((g.sp + 31) / 32), 32, 0, st>>>(s, g, ph, rk, nl, nullptr);
-  k_cn_back<><<<dim3((unsigned)((2 * g.sp + 127) / 128), 4), 128, 0, st>>>(s, g, nl, nullptr);
+  return go_cn_solve<false>(g, ph, s, rk, nl, nullptr, 1, st);
+}
+template <bool B>
+static cudaError_t go_tri_coef(const Geom& g, const Phys& ph, TriRow* tri, CnRow* cnr, DevScalars* sc, int rk, const MemberArgs* tab,
+                               int n, cudaStream_t st) {
+  const size_t smem = (size_t)g.np * sizeof(double2);
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(k_tri_lu<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e) return e;
+  }
+  k_tri_rows<B><<<dim3(4, n), 256, 0, st>>>(g, ph, tri, cnr, sc, rk, tab);
+  k_tri_lu<B><<<dim3(4, n), 256, smem, st>>>(g.np, cn_chunks(g), tri, cnr, tab);
   return cudaGetLastError();
 }
 cudaError_t launch_tri_coef(const Geom& g, const Phys& ph, const State& s, int rk, cudaStream_t st) {
-  const size_t smem = (size_t)g.np * sizeof(TriRow);
-  if (smem > 48 * 1024) cudaFuncSetAttribute(k_tri_coef<>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  k_tri_coef<><<<4, 256, smem, st>>>(g, ph, s.tri, s.sc, rk, nullptr);
-  return cudaGetLastError();
+  return go_tri_coef<false>(g, ph, s.tri, s.cnr, s.sc, rk, nullptr, 1, st);
 }
 cudaError_t launch_courant(const Geom& g, const Phys& ph, const State& s, CflCtl ctl, cudaStream_t st) {
   const dim3 grid(16, 74);   // x: within a row, y: rows
@@ -1361,11 +1818,35 @@ cudaError_t launch_courant_final(const Phys& ph, const State& s, CflCtl ctl, cud
   k_courant_final<<<1, 1, 0, st>>>(s.sc, ph, ctl);
   return cudaGetLastError();
 }
-cudaError_t launch_rem_div(const Geom& g, const State& s, int rk, int update_cp, cudaStream_t st) {
-  const dim3 grid((2 * (g.nkx + 1) + 127) / 128, g.nkzp);
-  if ((long long)grid.x * grid.y > 6LL * sm_count()) k_rem_div<3, 7><<<grid, 128, 0, st>>>(s, g, rk, update_cp, nullptr);
-  else k_rem_div<4, 6><<<grid, 128, 0, st>>>(s, g, rk, update_cp, nullptr);
+template <int M, int CHN, bool B>
+static cudaError_t go_rem_div_t(const Geom& g, const State& s, int rk, int update_cp, const MemberArgs* tab, int n,
+                                cudaStream_t st) {
+  const size_t smem = rem_div_smem<M, CHN>(g.np);
+  const cudaError_t e = cudaFuncSetAttribute(k_rem_div_ch<M, CHN, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e) return e;
+  k_rem_div_ch<M, CHN, B><<<dim3((unsigned)((g.sp + M - 1) / M), n), CHN * M, smem, st>>>(s, g, rk, update_cp, tab);
   return cudaGetLastError();
+}
+template <bool B>
+static cudaError_t go_rem_div(const Geom& g, const State& s, int rk, int update_cp, const MemberArgs* tab, int n,
+                              cudaStream_t st) {
+  // as cn_form; us a substep: 64x65x64 59 -> 6, 256x129x256 165 -> 91, 32
+  // channels of 128x65x128 329 -> 338 (wide CTAs; 517 with 8 modes) but alone
+  // 66 -> 23, 512x257x512 590 -> 785 (stays)
+  if (g.sp <= CH_MODES) {
+    if (rem_div_smem<32, 8>(g.np) <= 75 * 1024 && g.sp >= 32 * CH_CTAS)   // three CTAs an SM
+      return go_rem_div_t<32, 8, B>(g, s, rk, update_cp, tab, n, st);
+    if (rem_div_smem<8, 32>(g.np) <= SMEM_CTA) return go_rem_div_t<8, 32, B>(g, s, rk, update_cp, tab, n, st);
+  }
+  const dim3 grid((2 * (g.nkx + 1) + 127) / 128, g.nkzp, n);
+  if ((long long)grid.x * grid.y * n > 6LL * sm_count())
+    k_rem_div<3, 7, B><<<grid, 128, 0, st>>>(s, g, rk, update_cp, tab);
+  else
+    k_rem_div<4, 6, B><<<grid, 128, 0, st>>>(s, g, rk, update_cp, tab);
+  return cudaGetLastError();
+}
+cudaError_t launch_rem_div(const Geom& g, const State& s, int rk, int update_cp, cudaStream_t st) {
+  return go_rem_div<false>(g, s, rk, update_cp, nullptr, 1, st);
 }
 cudaError_t launch_pfac(const Geom& g, const State& s, cudaStream_t st) {
   k_pfac<<<dim3((g.nkx + 1 + 127) / 128, g.nkzp), 128, 0, st>>>(g, s.pfac);
@@ -1460,10 +1941,7 @@ cudaError_t launch_substep_batch(const Geom& g, const Batch& b, int rk, cudaStre
   // the implicit systems' rows on the side stream, joined before the solves
   if ((e = cudaEventRecord(ev_fork, st))) return e;
   if ((e = cudaStreamWaitEvent(st_side, ev_fork, 0))) return e;
-  const size_t tsm = (size_t)g.np * sizeof(TriRow);
-  if (tsm > 48 * 1024) cudaFuncSetAttribute(k_tri_coef<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm);
-  k_tri_coef<true><<<dim3(4, bt.n), 256, tsm, st_side>>>(g, Phys{}, nullptr, nullptr, rk, bt.tab);
-  if ((e = cudaGetLastError())) return e;
+  if ((e = go_tri_coef<true>(g, Phys{}, nullptr, nullptr, nullptr, rk, bt.tab, bt.n, st_side))) return e;
   if ((e = cudaEventRecord(ev_join, st_side))) return e;
   // velocity and buoyancy to physical space, products, z-pass of the products
   bt.nf = 4; bt.fin = FS_CU4; bt.fout = FS_XH4;
@@ -1490,16 +1968,8 @@ cudaError_t launch_substep_batch(const Geom& g, const Batch& b, int rk, cudaStre
   }
   // spectral RHS + CN solves, projection
   if ((e = cudaStreamWaitEvent(st, ev_join, 0))) return e;
-  const dim3 gr((unsigned)((g.sp + 31) / 32), bt.n);
-  if (!g.prec) k_rhs_cn<true, true><<<gr, 32, 0, st>>>(State{}, g, Phys{}, rk, FieldSet{}, bt.tab);
-  else k_rhs_cn<false, true><<<gr, 32, 0, st>>>(State{}, g, Phys{}, rk, FieldSet{}, bt.tab);
-  k_cn_back<true><<<dim3((unsigned)((2 * g.sp + 127) / 128), 4, bt.n), 128, 0, st>>>(State{}, g, FieldSet{}, bt.tab);
-  const dim3 grd((2 * (g.nkx + 1) + 127) / 128, g.nkzp, bt.n);
-  if ((long long)grd.x * grd.y * grd.z > 6LL * sm_count())
-    k_rem_div<3, 7, true><<<grd, 128, 0, st>>>(State{}, g, rk, 1, bt.tab);
-  else
-    k_rem_div<4, 6, true><<<grd, 128, 0, st>>>(State{}, g, rk, 1, bt.tab);
-  return cudaGetLastError();
+  if ((e = go_cn_solve<true>(g, Phys{}, State{}, rk, FieldSet{}, bt.tab, bt.n, st))) return e;
+  return go_rem_div<true>(g, State{}, rk, 1, bt.tab, bt.n, st);
 }
 
 }  // namespace db
