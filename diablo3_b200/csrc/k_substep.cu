@@ -25,6 +25,8 @@
 // The CN solves with eddy viscosity (one matrix per column) are in k_les.cu.
 #include <math.h>
 
+#include <type_traits>
+
 #include "../../include/diablo_b200.h"
 #include "db_bc.cuh"
 #include "db_kernels.cuh"
@@ -108,33 +110,54 @@ __device__ __forceinline__ void prod_ab(const ProdRows<R>& P, int grp, int seq, 
   }
 }
 
+// calls f<group, sequence> of a run-time pair that is the same for a whole warp
+// (one branch per sequence; inside the element loops it cost a branch per
+// element and most of the products kernels' instructions)
+template <typename F>
+__device__ __forceinline__ void with_seq(int grp, int seq, F&& f) {
+  if (grp == 0) {
+    if (seq == 0) f(std::integral_constant<int, 0>{}, std::integral_constant<int, 0>{});
+    else if (seq == 1) f(std::integral_constant<int, 0>{}, std::integral_constant<int, 1>{});
+    else f(std::integral_constant<int, 0>{}, std::integral_constant<int, 2>{});
+  } else {
+    if (seq == 0) f(std::integral_constant<int, 1>{}, std::integral_constant<int, 0>{});
+    else if (seq == 1) f(std::integral_constant<int, 1>{}, std::integral_constant<int, 1>{});
+    else f(std::integral_constant<int, 1>{}, std::integral_constant<int, 2>{});
+  }
+}
+
 // outputs of one transformed sequence (in sq, natural order), scaled by
 // 1/Nx: an N-type output ikx X(a) + X(b), and for s1 (group 0) / s2 (both
 // groups) the parts
 template <int N, typename C>
-__device__ __forceinline__ void prod_out(C* const* xh, const C* sq, const Geom& g, long long hrow, int grp, int seq,
+__device__ __forceinline__ void prod_out(C* const* xh, const C* sq, const Geom& g, long long hrow, int grp0, int seq0,
                                          int lane, bool r2, bool rt) {
   using R = typename RealOf<C>::type;
   constexpr int T = FftShape<N>::T;
   const R sc = (R)(1.0 / (double)N);
-  const bool n_out = (seq < 2) ? ((grp == 0) || (seq == 0 ? r2 : rt)) : false;
-  const int o_n = (grp == 0) ? (seq == 0 ? 0 : 2) : (seq == 0 ? 4 : 6);
   const C Z = mkc<C>(0, 0);
-  for (int mm = lane; mm < g.kxs; mm += T) {
-    const bool live = mm <= g.nkx;
-    const C A = live ? sepp<N>(sq, mm, 0) : Z;
-    const C B = live ? sepp<N>(sq, mm, 1) : Z;
-    if (seq < 2) {
-      const R k = (R)g.kx[mm];
-      xh[o_n][hrow + mm] = n_out ? mkc<C>((B.x - k * A.y) * sc, (B.y + k * A.x) * sc) : Z;
+  with_seq(grp0, seq0, [&](auto G_, auto S_) {
+    constexpr int grp = decltype(G_)::value, seq = decltype(S_)::value;
+    const bool n_out = (seq < 2) ? ((grp == 0) || (seq == 0 ? r2 : rt)) : false;
+    constexpr int o_n = (grp == 0) ? (seq == 0 ? 0 : 2) : (seq == 0 ? 4 : 6);
+    C* const pn = xh[o_n] + hrow;                                              // N of s0, s1
+    C* const pa = xh[grp == 0 ? (seq == 1 ? 1 : 3) : 5] + hrow;                // M1, M3, M2
+    C* const pb = xh[7] + hrow;                                                // MT
+    for (int mm = lane; mm < g.kxs; mm += T) {
+      const bool live = mm <= g.nkx;
+      const C A = live ? sepp<N>(sq, mm, 0) : Z;
+      const C B = live ? sepp<N>(sq, mm, 1) : Z;
+      if (seq < 2) {
+        const R k = (R)g.kx[mm];
+        pn[mm] = n_out ? mkc<C>((B.x - k * A.y) * sc, (B.y + k * A.x) * sc) : Z;
+      }
+      if (grp == 0 && seq >= 1) pa[mm] = mkc<C>(A.x * sc, A.y * sc);   // M1, M3
+      if (grp == 1 && seq == 2) {
+        pa[mm] = r2 ? mkc<C>(A.x * sc, A.y * sc) : Z;  // M2
+        pb[mm] = rt ? mkc<C>(B.x * sc, B.y * sc) : Z;  // MT
+      }
     }
-    if (grp == 0 && seq == 1) xh[1][hrow + mm] = mkc<C>(A.x * sc, A.y * sc);       // M1
-    if (grp == 0 && seq == 2) xh[3][hrow + mm] = mkc<C>(A.x * sc, A.y * sc);       // M3
-    if (grp == 1 && seq == 2) {
-      xh[5][hrow + mm] = r2 ? mkc<C>(A.x * sc, A.y * sc) : Z;  // M2
-      xh[7][hrow + mm] = rt ? mkc<C>(B.x * sc, B.y * sc) : Z;  // MT
-    }
-  }
+  });
 }
 
 // One CTA per (z, j, group), rows read from global memory (Nx > 512).
@@ -197,7 +220,10 @@ __global__ void __launch_bounds__(3 * FftShape<N>::T, FftShape<N>::T >= 128 ? 1 
 //        overlapping the second group's FFT and the next plane's first
 //        group.  With an exchange stride of padded(N) - 1 a CTA holds
 //        < 76 KB of shared memory, and three CTAs share an SM.
-// Thread layout: sequence (zi, seq) = (sidx / 3, sidx % 3).
+// Bound by instructions (IPC 2 of 4, DRAM at 8 to 15 %): with the group and
+// sequence branches out of the element loops, one sequence per warp, and three
+// CTAs of the persistent FP32 grid, us a substep 512x257x512 4129 -> 3735
+// (FP64) and 3614 -> 2678 (FP32), 32 channels of 128x65x128 1494 -> 1227.
 template <typename R>
 constexpr int prod_slots() { return sizeof(R) == sizeof(double) ? 4 : 3; }
 constexpr uint32_t PROD_WAIT = 1u << 24;
@@ -225,8 +251,10 @@ __global__ void __launch_bounds__(192, prod_slots<R>() == 4 ? 2 : 3) k_products_
   constexpr int PROD_SLOTS = prod_slots<R>();
   C* xbuf = reinterpret_cast<C*>(sm_raw + PROD_SLOTS * slot_bytes);
   uint64_t* mbar = reinterpret_cast<uint64_t*>(sm_raw + PROD_SLOTS * slot_bytes + (size_t)3 * zr * SQ * sizeof(C));
+  // the CTA's first third holds sequence 0 of its rows, and so on, so that a
+  // warp holds one sequence where zr T >= 32
   const int sidx = threadIdx.x / T, lane = threadIdx.x % T;
-  const int zi = sidx / 3, seq = sidx % 3;
+  const int zi = sidx % zr, seq = sidx / zr;
   C* sq = xbuf + sidx * SQ;
   const C* twt = tw_x<R>(g);
   C* const* xh = reinterpret_cast<C* const*>(s.xh);
@@ -298,12 +326,14 @@ __global__ void __launch_bounds__(192, prod_slots<R>() == 4 ? 2 : 3) k_products_
           const int jm = j >= 1 ? j - 1 : j, jp = j + 1 <= np - 1 ? j + 1 : j;
           const ProdRows<R> P{row(jm, 0), row(j, 0), row(jp, 0), row(jm, 1), row(j, 1), row(jp, 1),
                               row(jm, 2), row(j, 2), row(jp, 2), row(jm, 3), row(j, 3), row(jp, 3)};
+          with_seq(grp, seq, [&](auto G_, auto S_) {
 #pragma unroll
-          for (int q = 0; q < E; ++q) {
-            R a, b;
-            prod_ab(P, grp, seq, lane + q * T, r2, rt, y, a, b);
-            v[q] = mkc<C>(a, b);
-          }
+            for (int q = 0; q < E; ++q) {
+              R a, b;
+              prod_ab(P, decltype(G_)::value, decltype(S_)::value, lane + q * T, r2, rt, y, a, b);
+              v[q] = mkc<C>(a, b);
+            }
+          });
         }
         if (PROD_SLOTS == 3 && grp == 1) {   // plane j - 1 is read for the last time: its slot takes plane j + 2
           __syncthreads();
@@ -340,7 +370,7 @@ __global__ void __launch_bounds__(3 * FftShape<N>::T * prod_zr<N>()) k_products_
   constexpr int E = S::E, T = S::T;
   extern __shared__ __align__(16) unsigned char sm_raw[];
   const int sidx = threadIdx.x / T, lane = threadIdx.x % T;
-  const int zi = sidx / 3, seq = sidx % 3;
+  const int zi = sidx % zr, seq = sidx / zr;   // as k_products_st
   const int z0 = blockIdx.x * zr, z = z0 + zi, j = blockIdx.y, grp = blockIdx.z;
   const bool r1 = in_rng(j, g.jstart, g.jend);
   const bool r2 = in_rng(j, 2, g.ny);
@@ -1647,7 +1677,7 @@ static void go_products_t(const Geom& g, const State& s, cudaStream_t st) {
     if (smem > 48 * 1024)
       cudaFuncSetAttribute(k_products_st<N, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     const int nzb = g.nz / zr;
-    const int gmax = (g.tune_pgrid > 0 ? g.tune_pgrid : 2) * sm_count();
+    const int gmax = (g.tune_pgrid > 0 ? g.tune_pgrid : (PROD_SLOTS == 4 ? 2 : 3)) * sm_count();
     // plane ranges: about four items per CTA, at least four planes each
     int nch = (4 * gmax + nzb - 1) / nzb;
     nch = nch < 1 ? 1 : (nch > g.np / 4 ? (g.np / 4 > 0 ? g.np / 4 : 1) : nch);
