@@ -787,11 +787,10 @@ extern "C" int db_fft_xz_to_physical(db_ctx* c, double* buf) {
 extern "C" int db_fft_xz_to_fourier_dev(db_ctx* c, double* d) {
   if (!c || !d) return DB_ERR_ARG;
   const Geom& g = c->g;
-  CK(launch_phys_from_ref(g, c->p.nx, c->p.nz, d, c->s.r1, c->st));
-  CK(launch_fwd_x(g, fset(c->s.r1), fset(c->s.xh[0]), 1, c->st));
+  CK(launch_fwd_x_ref(g, d, c->s.xh[0], c->st));
   CK(launch_fwd_z(g, fset(c->s.xh[0]), fset(c->s.phi_g), 1, c->st));
   CK(launch_spec_to_ref(g, c->p.nx, c->p.nz, c->s.phi_g, reinterpret_cast<double2*>(d), c->st));
-  c->launches += 4;
+  c->launches += 3;
   return DB_OK;
 }
 
@@ -800,9 +799,8 @@ extern "C" int db_fft_xz_to_physical_dev(db_ctx* c, double* d) {
   const Geom& g = c->g;
   CK(launch_ref_to_spec(g, c->p.nx, c->p.nz, reinterpret_cast<const double2*>(d), c->s.phi_g, c->st));
   CK(launch_inv_z(g, fset(c->s.phi_g), fset(c->s.xh[0]), 1, c->st));
-  CK(launch_inv_x(g, fset(c->s.xh[0]), fset(c->s.r1), 1, c->st));
-  CK(launch_phys_to_ref(g, c->p.nx, c->p.nz, c->s.r1, d, c->st));
-  c->launches += 4;
+  CK(launch_inv_x_ref(g, c->s.xh[0], d, c->st));
+  c->launches += 3;
   return DB_OK;
 }
 

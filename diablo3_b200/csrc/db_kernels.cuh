@@ -52,6 +52,10 @@ inline FieldSet fset(void* a = nullptr, void* b = nullptr, void* c = nullptr, vo
 
 // k_fft.cu
 cudaError_t launch_fwd_x(const Geom& g, FieldSet in, FieldSet out, int nf, cudaStream_t st);
+// the x-pass of one field whose physical side is a device array in the
+// reference layout (FP64, 16-byte aligned)
+cudaError_t launch_fwd_x_ref(const Geom& g, const double* ref, void* xh, cudaStream_t st);
+cudaError_t launch_inv_x_ref(const Geom& g, void* xh, double* ref, cudaStream_t st);
 // dmask: bit f set -> field f is differentiated (x: i kx, z: i kz) on the way
 cudaError_t launch_inv_x(const Geom& g, FieldSet in, FieldSet out, int nf, cudaStream_t st, unsigned dmask = 0);
 // accumulate: out += transform, with rows 0, 1, Nyp, Nyp+1 based on ghost
@@ -253,10 +257,6 @@ cudaError_t launch_stats(const Geom& g, const State& s, int homx, double* out, c
 // spectral field: compact device layout <-> reference host layout, on the device
 cudaError_t launch_spec_to_ref(const Geom& g, int nx, int nz, const double2* src, double2* ref, cudaStream_t st);
 cudaError_t launch_ref_to_spec(const Geom& g, int nx, int nz, const double2* ref, double2* dst, cudaStream_t st);
-// one physical field between the reference layout (device doubles) and the
-// compact layout at the context's precision
-cudaError_t launch_phys_from_ref(const Geom& g, int nx, int nz, const double* ref, void* dst, cudaStream_t st);
-cudaError_t launch_phys_to_ref(const Geom& g, int nx, int nz, const void* src, double* ref, cudaStream_t st);
 cudaError_t launch_bc_vel_post(const Geom& g, const Phys& ph, const State& s, cudaStream_t st);
 
 // k_les.cu

@@ -16,6 +16,8 @@
 // R is the real type of the physical and x-half fields: double, or float on
 // the mixed path, where the spectral state stays FP64 and is converted on
 // the z-pass load/store.
+#include <type_traits>
+
 #include "../../include/diablo_b200.h"
 #include "db_kernels.cuh"
 #include "fft_reg.cuh"
@@ -334,27 +336,34 @@ __global__ void __launch_bounds__(256, DB_LB_FFT) k_inv_z(const __grid_constant_
 // contiguous, so one thread brings the NEXT item's rows into the other half
 // of a double buffer with a single cp.async.bulk while the CTA transforms the
 // current item from shared memory: the load latency hides behind the FFT.
+// REF: the physical side is a field in the reference layout, FP64 rows of
+// Nx + 2 (0:Nx+1, 0:Nz+1, 0:Nyp+1); the padding is staged with the rows on the
+// way in and not written on the way out.  (A layout pass before the forward
+// and after the inverse transform cost 131 and 154 us of 885 at 512x129x512.)
 constexpr uint32_t STAGE_WAIT = 1u << 24;
 
-template <int N, typename R>
+template <int N, typename R, bool REF = false>
 __global__ void __launch_bounds__(256, 2) k_fwd_x_st(const __grid_constant__ FieldSet in, const __grid_constant__ FieldSet out, Geom g, int nblk,
                                                      int nitems) {
   using C = typename CplxOf<R>::type;
+  using I = typename std::conditional<REF, double, R>::type;   // stored type of the rows
+  constexpr int P = REF ? N + 2 : N;                           // and their pitch
   using S = FftShape<N>;
   constexpr int E = S::E, T = S::T;
   extern __shared__ __align__(16) unsigned char sm_raw[];
   const int ns = blockDim.x / T;                       // sequences (row pairs) per item
-  const uint32_t row_bytes = N * sizeof(R);
+  const uint32_t row_bytes = P * sizeof(I);
   const uint32_t item_bytes = 2u * ns * row_bytes;
-  R* stage0 = reinterpret_cast<R*>(sm_raw);
+  I* stage0 = reinterpret_cast<I*>(sm_raw);
   C* xbuf = reinterpret_cast<C*>(sm_raw + 2 * item_bytes);
   uint64_t* mbar = reinterpret_cast<uint64_t*>(sm_raw + 2 * item_bytes + (size_t)ns * padded(N) * sizeof(C));
   const int seq = threadIdx.x / T, lane = threadIdx.x % T;
   C* sq = xbuf + seq * padded(N);
   const C* twt = tw_x<R>(g);   // twiddles fetched per pass (fewer live registers)
-  auto src = [&](int it) -> const R* {
+  auto src = [&](int it) -> const I* {
     const int f = it / (g.np * nblk), r = it % (g.np * nblk), j = r / nblk, b = r % nblk;
-    return (const R*)in.p[f] + (long long)j * g.pp + (long long)(2 * ns * b) * g.nx;
+    if (REF) return (const I*)in.p[f] + ((long long)j * (g.nz + 2) + 2 * ns * b) * P;
+    return (const I*)in.p[f] + (long long)j * g.pp + (long long)(2 * ns * b) * g.nx;
   };
   if (threadIdx.x == 0) {
     mbar_init(&mbar[0], 1);
@@ -384,12 +393,12 @@ __global__ void __launch_bounds__(256, 2) k_fwd_x_st(const __grid_constant__ Fie
       }
       return;
     }
-    const R* ra = reinterpret_cast<const R*>(reinterpret_cast<const unsigned char*>(stage0) + s * item_bytes) +
-                  (2 * seq) * N;
-    const R* rb = ra + N;
+    const I* ra = reinterpret_cast<const I*>(reinterpret_cast<const unsigned char*>(stage0) + s * item_bytes) +
+                  (2 * seq) * P;
+    const I* rb = ra + P;
     C v[E];
 #pragma unroll
-    for (int q = 0; q < E; ++q) v[q] = mkc<C>(ra[lane + q * T], rb[lane + q * T]);
+    for (int q = 0; q < E; ++q) v[q] = mkc<C>((R)ra[lane + q * T], (R)rb[lane + q * T]);
     fft_reg_lazy<N, -1>(v, lane, true, sq, twt);
     SEQ_SYNC(N);
 #pragma unroll
@@ -429,7 +438,7 @@ struct CflArgs {
 // B: member-batched (the persistent CTAs walk the items of every member,
 // member = item / nitems; g is member 0's geometry, the same for all; no
 // dmask, not with CFL)
-template <int N, typename R, bool CFL, bool B = false>
+template <int N, typename R, bool CFL, bool B = false, bool REF = false>
 __global__ void __launch_bounds__(256, 2) k_inv_x_st(const __grid_constant__ FieldSet in, const __grid_constant__ FieldSet out, Geom g,
                                                       unsigned dmask, int nblk, int nitems,
                                                       const __grid_constant__ CflArgs cf, const __grid_constant__ Batch bt) {
@@ -539,12 +548,14 @@ __global__ void __launch_bounds__(256, 2) k_inv_x_st(const __grid_constant__ Fie
         amax = fmax(amax, fmax(ta, tb));
       }
     } else {
-      R* ra = (R*)fs_out(it).p[f] + (long long)j * g.pp + (long long)(2 * (ns * b + seq)) * g.nx;
-      R* rb = ra + g.nx;
+      using O = typename std::conditional<REF, double, R>::type;
+      const int z = 2 * (ns * b + seq);
+      O* ra = (O*)fs_out(it).p[f] + (REF ? ((long long)j * (g.nz + 2) + z) * (N + 2) : (long long)j * g.pp + (long long)z * g.nx);
+      O* rb = ra + (REF ? N + 2 : N);
 #pragma unroll
       for (int q = 0; q < E; ++q) {
-        ra[lane + q * T] = v[q].x;
-        rb[lane + q * T] = v[q].y;
+        ra[lane + q * T] = (O)v[q].x;
+        rb[lane + q * T] = (O)v[q].y;
       }
     }
     __syncthreads();
@@ -617,27 +628,28 @@ int sm_count() {
   return n;
 }
 
-template <int N, typename R>
+template <int N, typename R, bool REF = false>
 static void go_fwd_x_t(const Geom& g, FieldSet in, FieldSet out, int nf, cudaStream_t st) {
   using C = typename CplxOf<R>::type;
   const int cps = xpass_cps<N>(g);
   const int nblk = (g.nz / 2) / cps, nitems = nblk * g.np * nf;
-  const size_t smem = 2 * (size_t)(2 * cps * N * sizeof(R)) + (size_t)cps * padded(N) * sizeof(C) + 16;
-  smem_attr(k_fwd_x_st<N, R>, smem);
+  const size_t row = REF ? (N + 2) * sizeof(double) : N * sizeof(R);
+  const size_t smem = 2 * (2 * cps * row) + (size_t)cps * padded(N) * sizeof(C) + 16;
+  smem_attr(k_fwd_x_st<N, R, REF>, smem);
   const int gmax = xpass_ctas_per_sm(g) * sm_count();
   const int grid = nitems < gmax ? nitems : gmax;
-  k_fwd_x_st<N, R><<<grid, cps * FftShape<N>::T, smem, st>>>(in, out, g, nblk, nitems);
+  k_fwd_x_st<N, R, REF><<<grid, cps * FftShape<N>::T, smem, st>>>(in, out, g, nblk, nitems);
 }
-template <int N, typename R>
+template <int N, typename R, bool REF = false>
 static void go_inv_x_t(const Geom& g, FieldSet in, FieldSet out, int nf, unsigned dmask, cudaStream_t st) {
   using C = typename CplxOf<R>::type;
   const int cps = xpass_cps<N>(g);
   const int nblk = (g.nz / 2) / cps, nitems = nblk * g.np * nf;
   const size_t smem = 2 * (size_t)(2 * cps * g.kxs * sizeof(C)) + (size_t)cps * padded(N) * sizeof(C) + 16;
-  smem_attr(k_inv_x_st<N, R, false>, smem);
+  smem_attr(k_inv_x_st<N, R, false, false, REF>, smem);
   const int gmax = xpass_ctas_per_sm(g) * sm_count();
   const int grid = nitems < gmax ? nitems : gmax;
-  k_inv_x_st<N, R, false><<<grid, cps * FftShape<N>::T, smem, st>>>(in, out, g, dmask, nblk, nitems, CflArgs{}, Batch{});
+  k_inv_x_st<N, R, false, false, REF><<<grid, cps * FftShape<N>::T, smem, st>>>(in, out, g, dmask, nblk, nitems, CflArgs{}, Batch{});
 }
 template <int N, typename R>
 static void go_inv_x_cfl_t(const Geom& g, FieldSet in, const CflArgs& cf, cudaStream_t st) {
@@ -717,6 +729,24 @@ static void go_inv_z(const Geom& g, FieldSet in, FieldSet out, int nf, unsigned 
   else go_inv_z_t<N, double>(g, in, out, nf, dmask, ghost, mean, st);
 }
 
+template <int N>
+static void go_fwd_x_ref(const Geom& g, FieldSet in, FieldSet out, cudaStream_t st) {
+  if (g.prec) go_fwd_x_t<N, float, true>(g, in, out, 1, st);
+  else go_fwd_x_t<N, double, true>(g, in, out, 1, st);
+}
+template <int N>
+static void go_inv_x_ref(const Geom& g, FieldSet in, FieldSet out, cudaStream_t st) {
+  if (g.prec) go_inv_x_t<N, float, true>(g, in, out, 1, 0u, st);
+  else go_inv_x_t<N, double, true>(g, in, out, 1, 0u, st);
+}
+cudaError_t launch_fwd_x_ref(const Geom& g, const double* ref, void* xh, cudaStream_t st) {
+  DB_DISPATCH_N(g.nx, go_fwd_x_ref, g, fset(const_cast<double*>(ref)), fset(xh), st);
+  return cudaGetLastError();
+}
+cudaError_t launch_inv_x_ref(const Geom& g, void* xh, double* ref, cudaStream_t st) {
+  DB_DISPATCH_N(g.nx, go_inv_x_ref, g, fset(xh), fset(ref), st);
+  return cudaGetLastError();
+}
 cudaError_t launch_fwd_x(const Geom& g, FieldSet in, FieldSet out, int nf, cudaStream_t st) {
   if (nf < 1 || nf > MAXF) return cudaErrorInvalidValue;
   DB_DISPATCH_N(g.nx, go_fwd_x, g, in, out, nf, st);
