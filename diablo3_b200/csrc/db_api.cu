@@ -169,10 +169,15 @@ static void twiddles_f(int n, std::vector<float2>& out) {
 static size_t phys_elem(const db_ctx* c) { return c->p.precision ? sizeof(float) : sizeof(double); }
 static size_t xh_elem(const db_ctx* c) { return c->p.precision ? sizeof(float2) : sizeof(double2); }
 
+// (The zeros are written on the context's stream and waited for: a plain
+// cudaMemset runs on the legacy stream, which neither the context's
+// non-blocking stream nor the host waits for, and could land on top of what
+// the caller puts into the new buffer next.)
 static int balloc(db_ctx* c, void** ptr, size_t bytes) {
   void* q = nullptr;
   CK(cudaMalloc(&q, bytes));
-  CK(cudaMemset(q, 0, bytes));
+  CK(cudaMemsetAsync(q, 0, bytes, c->st));
+  CK(cudaStreamSynchronize(c->st));
   c->allocs.push_back(q);
   *ptr = q;
   return DB_OK;
@@ -182,7 +187,8 @@ template <typename T>
 static int dalloc(db_ctx* c, T** ptr, size_t count) {
   void* q = nullptr;
   CK(cudaMalloc(&q, count * sizeof(T)));
-  CK(cudaMemset(q, 0, count * sizeof(T)));
+  CK(cudaMemsetAsync(q, 0, count * sizeof(T), c->st));
+  CK(cudaStreamSynchronize(c->st));
   c->allocs.push_back(q);
   *ptr = (T*)q;
   return DB_OK;
@@ -427,7 +433,10 @@ static int init_impl(const db_params* p, const double* gy_in, void* stream, db_c
     g_init_err = "db_init: pinned staging allocation failed";
     return DB_ERR_CUDA;
   }
-  if (launch_pfac(g, s, c->st) != cudaSuccess || cudaStreamSynchronize(c->st) != cudaSuccess) {
+  // the tables above went up on the legacy stream, from pageable memory: wait
+  // for their last bytes before the context's stream reads them
+  if (cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess || launch_pfac(g, s, c->st) != cudaSuccess ||
+      cudaStreamSynchronize(c->st) != cudaSuccess) {
     g_init_err = std::string("db_init: ") + cudaGetErrorString(cudaGetLastError());
     db_finalize(c);
     return DB_ERR_CUDA;
