@@ -857,6 +857,74 @@ __global__ void __launch_bounds__(256) k_tri_lu(int np, int ch, TriRow* tri0, Cn
 // mode are two real columns of the same real system, with the LU factors
 // k_tri_lu leaves.
 //
+// r + a v, r + i a v
+__device__ __forceinline__ double2 axpy(double2 r, double a, double2 v) {
+  return make_double2(r.x + a * v.x, r.y + a * v.y);
+}
+__device__ __forceinline__ double2 axpy_i(double2 r, double a, double2 v) {
+  return make_double2(r.x - a * v.y, r.y + a * v.x);
+}
+
+// The constants of one mode in the right-hand sides below.
+struct CnMode {
+  double nk, nkt, qt, gb, kxp, kzq, fx, kzv, temp3, temp5, f, c1, c3;
+};
+__device__ __forceinline__ CnMode cn_mode(const State& s, const Geom& g, const Phys& ph, int rk, int kx, int kzp) {
+  const RhsK kc = rhs_consts(s, g, ph, rk, kx, kzp);
+  const bool m0 = kx == 0 && kzp == 0;
+  const double tw = ph.front_tw ? ph.delta / ph.ro_inv : 0.0;   // thermal wind of the front
+  CnMode k;
+  k.f = ph.ro_inv / ph.delta;
+  k.qt = tw * (ph.dthdx * kc.kzv - ph.dthdz * kc.kxv);
+  k.c1 = -(ph.dthdz * tw);
+  k.c3 = ph.dthdx * tw;
+  k.nk = -ph.nu * kc.kk;
+  k.nkt = -(ph.nu / ph.pr) * kc.kk;
+  k.gb = m0 ? 0.0 : 1.0;   // no buoyancy in the mean u2 equation
+  k.kxp = -kc.temp4 * kc.kxv;
+  k.kzq = -kc.temp4 * kc.kzv;
+  k.kzv = kc.kzv;
+  k.temp3 = kc.temp3;
+  k.temp5 = kc.temp5;
+  k.fx = 0.0;   // mean forcing of u1
+  if (m0 && ph.f_type == 1) k.fx = -kc.temp4 * ph.px0;
+  if (m0 && ph.f_type == 2) k.fx = -kc.temp4 * (ph.px0 + ph.amp_omega0 * cos(ph.omega0 * s.sc->time));
+  return k;
+}
+// Right-hand side of equation e on row j: cf (solver.f90:396-609, 35-111), cr
+// (824-838, 966-973) and the explicit CN term (850-870, 981-989), from the
+// state of planes j-1, j, j+1 (um, u, un; order u1, u3, u2, th), v2 = <u2>,
+// cp of planes j and j-1, NL n (n + i kz z with SPLITZ) and the old cf h.
+// rhs_eval with the row's metric factors and the mode's products formed once:
+// its divisions and branches were two thirds of the solve's instructions
+// (k_rhs_cn at 512x257x512 1472 -> 1331 us a substep, mixed 1350 -> 1012).
+template <bool SPLITZ>
+__device__ __forceinline__ double2 cn_rhs(const CnRow& row, const CnMode& k, const Phys& ph, int e, const double2* um,
+                                          const double2* uc, double2 un, double2 v2, double2 cp, double2 pm, double2 n,
+                                          double2 z, double2 h, double sf, double sg, double2& cf) {
+  const double2 u = uc[e];
+  const double d = e == 3 ? k.nkt : k.nk;
+  cf = axpy_i(make_double2(u.x * d, u.y * d), -(e == 2 ? sg : sf), u);
+  if (e == 0) cf = axpy(axpy(axpy(cf, k.f, uc[1]), ph.grav_x, uc[3]), -k.c1, v2);
+  if (e == 1) cf = axpy(axpy(axpy(cf, -k.f, uc[0]), ph.grav_z, uc[3]), -k.c3, v2);
+  if (e == 2) cf = axpy(axpy(cf, k.gb * row.g[0], uc[3]), k.gb * row.g[1], um[3]);
+  if (e == 3) cf = axpy(axpy(cf, -ph.dthdx, uc[0]), -ph.dthdz, uc[1]);
+  cf.x -= n.x;
+  cf.y -= n.y;
+  if (SPLITZ) cf = axpy_i(cf, -k.kzv, z);   // NL = Z(N) + i kz Z(M), both already scaled by 1/Nz
+  double2 w = axpy(axpy(u, k.temp5, cf), k.temp3, h);
+  if (e == 0) {
+    w = axpy_i(w, k.kxp, cp);
+    w.x += k.fx;
+  }
+  if (e == 1) w = axpy_i(w, k.kzq, cp);
+  if (e == 2) w = axpy(w, -row.g[2], make_double2(cp.x - pm.x, cp.y - pm.y));
+  const double ch = row.cn[e][0], cl = row.cn[e][1];
+  w.x += ch * (un.x - u.x) - cl * (u.x - um[e].x);
+  w.y += ch * (un.y - u.y) - cl * (u.y - um[e].y);
+  return w;
+}
+
 // Two forms (cn_form): k_rhs_cn and k_cn_back walk all planes with one thread
 // per mode (many modes), k_cn_solve splits the planes into chunks.
 //
@@ -888,13 +956,12 @@ __global__ void __launch_bounds__(32, DB_RHSCN_LB) k_rhs_cn(const __grid_constan
   const int np = g.np;
   const long long sp = g.sp;
   const int kzp = m / g.kxs, kx = m % g.kxs;
-  const RhsK kc = rhs_consts(s, g, ph, rk, kx, kzp);
+  const CnMode k = cn_mode(s, g, ph, rk, kx, kzp);
   const bool m0 = (m == 0);   // the (0,0) mode carries the BC constants
   // z-pass order 0 u1, 1 u3, 2 u2, 3 th; k_tri_rows order th, u2, u1, u3
   const double2* const U[4] = {s.cu1 + m, s.cu3 + m, s.cu2 + m, s.cth + m};
   const int lo[4] = {g.jstart, g.jstart, 2, g.jstart_th};
   const int hi[4] = {g.jend, g.jend, g.ny, g.jend_th};
-  const TriRow* const Rw[4] = {s.tri + 2 * np, s.tri + 3 * np, s.tri + np, s.tri};
   double2 um[4], uc[4], y[4];
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
@@ -929,42 +996,20 @@ __global__ void __launch_bounds__(32, DB_RHSCN_LB) k_rhs_cn(const __grid_constan
       cfo[e] = (rr && rk > 0) ? rhs_cf(s, e)[a + m] : make_double2(0.0, 0.0);
     }
     const double2 cpj = s.cp[a + m];
-    if (SPLITZ) {   // NL = Z(N) + i kz Z(M), both already scaled by 1/Nz
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        nlv[e] = make_double2(nlv[e].x - kc.kzv * zmv[e].y, nlv[e].y + kc.kzv * zmv[e].x);
+    const CnRow& row = s.cnr[j];
+    double sf = 0.0, sg = 0.0;
+    if (ph.front_tw) {
+      sf = (g.gyf[j] - 0.5 * ph.ly) * k.qt;
+      sg = (g.gy[j] - 0.5 * ph.ly) * k.qt;
     }
+    const double2 v2 = make_double2(0.5 * (uc[2].x + un[2].x), 0.5 * (uc[2].y + un[2].y));
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const TriRow* row = Rw[e] + j;
-      double2 cr = make_double2(0.0, 0.0);
-      if (in_rng(j, lo[e], hi[e])) {
-        RhsIn v;
-        v.own = uc[e];
-        v.cu1 = uc[0];
-        v.cu3 = uc[1];
-        v.cth = uc[3];
-        v.cp = cpj;
-        v.nb2 = (e == 2) ? um[3] : uc[2];   // u2: cth of plane j-1; u1, u3: cu2 of plane j
-        v.nbp = (e == 2) ? pm : un[2];      // u2: cp of plane j-1;  u1, u3: cu2 of plane j+1
-        v.cfo = cfo[e];
-        double2 cf;
-        cr = rhs_eval<false>(s, g, ph, rk, e, j, kx, kzp, nlv[e], v, kc, cf);
-        rhs_cf(s, e)[a + m] = cf;
-      }
-      double2 w;
-      if (row->is_bc) {
-        w = make_double2(m0 ? row->bc : 0.0, 0.0);
-      } else {
-        w.x = cr.x + (row->cn_hi * (un[e].x - uc[e].x) - row->cn_lo * (uc[e].x - um[e].x));
-        w.y = cr.y + (row->cn_hi * (un[e].y - uc[e].y) - row->cn_lo * (uc[e].y - um[e].y));
-      }
-      if (j == 0) {
-        y[e] = w;
-      } else {
-        y[e].x = w.x + row->ap * y[e].x;
-        y[e].y = w.y + row->ap * y[e].y;
-      }
+      double2 cf;
+      double2 w = cn_rhs<SPLITZ>(row, k, ph, e, um, uc, un[e], v2, cpj, pm, nlv[e], SPLITZ ? zmv[e] : cpj, cfo[e], sf, sg, cf);
+      if (in_rng(j, lo[e], hi[e])) rhs_cf(s, e)[a + m] = cf;
+      if (row.bc[e]) w = make_double2(m0 ? s.tri[(e == 0 ? 2 : e == 1 ? 3 : e == 2 ? 1 : 0) * np + j].bc : 0.0, 0.0);
+      y[e] = axpy(w, row.ap[e], y[e]);   // a' = 0 on row 0
       ((double2*)nl.p[e])[a + m] = y[e];
     }
 #pragma unroll
@@ -1089,14 +1134,6 @@ __device__ __forceinline__ void chunk_inflows(double2& y, double2& x, double p, 
   x.y = __shfl_sync(0xffffffffu, x.y, rc, CHN);
 }
 
-// r + a v, r + i a v
-__device__ __forceinline__ double2 axpy(double2 r, double a, double2 v) {
-  return make_double2(r.x + a * v.x, r.y + a * v.y);
-}
-__device__ __forceinline__ double2 axpy_i(double2 r, double a, double2 v) {
-  return make_double2(r.x - a * v.y, r.y + a * v.x);
-}
-
 template <int M, int CHN, bool SPLITZ, bool B = false>
 __global__ void __launch_bounds__(CHN * M) k_cn_solve(const __grid_constant__ State s0, Geom g0, Phys ph0, int rk,
                                                         const __grid_constant__ FieldSet nl0,
@@ -1131,18 +1168,8 @@ __global__ void __launch_bounds__(CHN * M) k_cn_solve(const __grid_constant__ St
     if (j0 < j1) {
       double2 x[4] = {Z2, Z2, Z2, Z2};
       const int kzp = (int)(m / g.kxs), kx = (int)(m % g.kxs);
-      const RhsK kc = rhs_consts(s, g, ph, rk, kx, kzp);
+      const CnMode k = cn_mode(s, g, ph, rk, kx, kzp);
       const bool m0 = (m == 0);   // the (0,0) mode carries the BC constants
-      const double f = ph.ro_inv / ph.delta;
-      const double tw = ph.front_tw ? ph.delta / ph.ro_inv : 0.0;   // thermal wind of the front
-      const double qt = tw * (ph.dthdx * kc.kzv - ph.dthdz * kc.kxv);
-      const double c1 = -(ph.dthdz * tw), c3 = ph.dthdx * tw;
-      const double nk = -ph.nu * kc.kk, nkt = -(ph.nu / ph.pr) * kc.kk;
-      const double gb = m0 ? 0.0 : 1.0;   // no buoyancy in the mean u2 equation
-      const double kxp = -kc.temp4 * kc.kxv, kzq = -kc.temp4 * kc.kzv;
-      double fx = 0.0;   // mean forcing of u1
-      if (m0 && ph.f_type == 1) fx = -kc.temp4 * ph.px0;
-      if (m0 && ph.f_type == 2) fx = -kc.temp4 * (ph.px0 + ph.amp_omega0 * cos(ph.omega0 * s.sc->time));
       const bool old = rk > 0;
       long long a = j0 * sp + m;
       double2 um[4], uc[4];
@@ -1170,38 +1197,16 @@ __global__ void __launch_bounds__(CHN * M) k_cn_solve(const __grid_constant__ St
         const CnRow& row = rows[j];
         double sf = 0.0, sg = 0.0;
         if (ph.front_tw) {
-          sf = (g.gyf[j] - 0.5 * ph.ly) * qt;
-          sg = (g.gy[j] - 0.5 * ph.ly) * qt;
+          sf = (g.gyf[j] - 0.5 * ph.ly) * k.qt;
+          sg = (g.gy[j] - 0.5 * ph.ly) * k.qt;
         }
         const double2 v2 = make_double2(0.5 * (uc[2].x + un[2].x), 0.5 * (uc[2].y + un[2].y));
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const bool rr = e < 2 ? rv : (e == 2 ? r2 : rt);
-          const double2 u = uc[e];
-          const double2 n = n4[e], h = h4[e], z = z4[e];
-          double2 w;
-          {
-            double2 cf = make_double2(u.x * (e == 3 ? nkt : nk), u.y * (e == 3 ? nkt : nk));
-            cf = axpy_i(cf, -(e == 2 ? sg : sf), u);
-            if (e == 0) cf = axpy(axpy(axpy(cf, f, uc[1]), ph.grav_x, uc[3]), -c1, v2);
-            if (e == 1) cf = axpy(axpy(axpy(cf, -f, uc[0]), ph.grav_z, uc[3]), -c3, v2);
-            if (e == 2) cf = axpy(axpy(cf, gb * row.g[0], uc[3]), gb * row.g[1], um[3]);
-            if (e == 3) cf = axpy(axpy(cf, -ph.dthdx, uc[0]), -ph.dthdz, uc[1]);
-            cf.x -= n.x;
-            cf.y -= n.y;
-            if (SPLITZ) cf = axpy_i(cf, -kc.kzv, z);   // NL = Z(N) + i kz Z(M), both already scaled by 1/Nz
-            if (rr) rhs_cf(s, e)[a] = cf;
-            w = axpy(axpy(u, kc.temp5, cf), kc.temp3, h);
-            if (e == 0) {
-              w = axpy_i(w, kxp, cp);
-              w.x += fx;
-            }
-            if (e == 1) w = axpy_i(w, kzq, cp);
-            if (e == 2) w = axpy(w, -row.g[2], make_double2(cp.x - pm.x, cp.y - pm.y));
-          }
-          const double ch = row.cn[e][0], cl = row.cn[e][1];
-          w.x += ch * (un[e].x - u.x) - cl * (u.x - um[e].x);
-          w.y += ch * (un[e].y - u.y) - cl * (u.y - um[e].y);
+          double2 cf;
+          double2 w = cn_rhs<SPLITZ>(row, k, ph, e, um, uc, un[e], v2, cp, pm, n4[e], z4[e], h4[e], sf, sg, cf);
+          if (rr) rhs_cf(s, e)[a] = cf;
           if (row.bc[e]) w = make_double2(m0 ? s.tri[(e == 0 ? 2 : e == 1 ? 3 : e == 2 ? 1 : 0) * np + j].bc : 0.0, 0.0);
           y[e] = axpy(w, row.ap[e], y[e]);   // a' = 0 on row 0
           ys[(j * 4 + e) * M + mi] = y[e];
