@@ -50,6 +50,16 @@ inline FieldSet fset(void* a = nullptr, void* b = nullptr, void* c = nullptr, vo
   return s;
 }
 
+// The limit on dynamic shared memory belongs to the kernel, not to a context:
+// every launcher asks for the same one, whatever its own sizes, so that a
+// context on another host thread cannot lower it between this call and the
+// launch.  fixed: the kernel's __shared__ variables, which share a CTA's 227 KB.
+constexpr size_t SMEM_CTA = 227 * 1024;
+template <typename K>
+cudaError_t smem_limit(K kern, size_t fixed = 0) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_CTA - fixed));
+}
+
 // k_fft.cu
 cudaError_t launch_fwd_x(const Geom& g, FieldSet in, FieldSet out, int nf, cudaStream_t st);
 // the x-pass of one field whose physical side is a device array in the

@@ -313,8 +313,8 @@ cudaError_t launch_bpe_pdf(const Geom& g, const Phys& ph, const double* th, int 
   const int nj = g.jend_th - g.jstart_th + 1;
   if (nj < 1 || nbin < 1) return cudaErrorInvalidValue;
   const size_t smem = (size_t)nbin * sizeof(double) * (fbin ? 2 : 1);
-  if (smem > 227 * 1024) return cudaErrorInvalidValue;
-  if (smem > 48 * 1024) cudaFuncSetAttribute(k_bpe_pdf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (smem > SMEM_CTA) return cudaErrorInvalidValue;
+  if (smem > 48 * 1024) smem_limit(k_bpe_pdf);
   k_bpe_pdf<<<dim3(8, nj), 256, smem, st>>>(th, g, ph, homx, nbin, pdf, fbin, kind, f0, f1, f2);
   return cudaGetLastError();
 }

@@ -597,8 +597,8 @@ constexpr int seqs_per_cta() {
   }
 
 template <typename K>
-static void smem_attr(K kern, size_t smem) {
-  if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+static void smem_attr(K kern, size_t smem, size_t fixed = 0) {
+  if (smem > 48 * 1024) smem_limit(kern, fixed);
 }
 
 // sequences per item of the staged x-pass: cps (<= seqs_per_cta, divides nz/2)
@@ -657,7 +657,7 @@ static void go_inv_x_cfl_t(const Geom& g, FieldSet in, const CflArgs& cf, cudaSt
   const int cps = xpass_cps<N>(g);
   const int nblk = (g.nz / 2) / cps, nitems = nblk * g.np * 3;
   const size_t smem = 2 * (size_t)(2 * cps * g.kxs * sizeof(C)) + (size_t)cps * padded(N) * sizeof(C) + 16;
-  smem_attr(k_inv_x_st<N, R, true>, smem);
+  smem_attr(k_inv_x_st<N, R, true>, smem, 32 * sizeof(double));   // its reduction
   const int gmax = xpass_ctas_per_sm(g) * sm_count();
   const int grid = nitems < gmax ? nitems : gmax;
   k_inv_x_st<N, R, true><<<grid, cps * FftShape<N>::T, smem, st>>>(in, FieldSet{}, g, 0u, nblk, nitems, cf, Batch{});

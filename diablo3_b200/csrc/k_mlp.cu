@@ -783,7 +783,8 @@ cudaError_t launch_adam(float* params, float* grads, float* m1, float* m2, int n
 cudaError_t launch_umma_gemm(const uint16_t* A, const uint16_t* B, float* D, int K, int N, int* err,
                              cudaStream_t st) {
   const size_t smem = (size_t)(128 + N) * K * 2 + 16;
-  cudaFuncSetAttribute(k_umma_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // the largest K and N: the same limit on every call (it belongs to the kernel)
+  cudaFuncSetAttribute(k_umma_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (128 + 256) * 256 * 2 + 16);
   k_umma_gemm<<<1, 128, smem, st>>>(A, B, D, K, N, err);
   return cudaGetLastError();
 }

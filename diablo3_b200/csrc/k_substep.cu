@@ -1679,8 +1679,7 @@ static void go_products_t(const Geom& g, const State& s, cudaStream_t st) {
     constexpr int PROD_SLOTS = prod_slots<R>();
     const size_t smem = (size_t)PROD_SLOTS * 4 * zr * N * sizeof(R) + (size_t)3 * zr * prod_sq<N>() * sizeof(C) +
                         PROD_SLOTS * sizeof(uint64_t);
-    if (smem > 48 * 1024)
-      cudaFuncSetAttribute(k_products_st<N, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) smem_limit(k_products_st<N, R>);
     const int nzb = g.nz / zr;
     const int gmax = (g.tune_pgrid > 0 ? g.tune_pgrid : (PROD_SLOTS == 4 ? 2 : 3)) * sm_count();
     // plane ranges: about four items per CTA, at least four planes each
@@ -1693,7 +1692,7 @@ static void go_products_t(const Geom& g, const State& s, cudaStream_t st) {
     k_products_st<N, R><<<grid, 3 * FftShape<N>::T * zr, smem, st>>>(s, g, zr, nzb, jlen, nitems, nullptr);
   } else {
     const size_t smem = (size_t)3 * padded(N) * sizeof(C);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_products<N, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) smem_limit(k_products<N, R>);
     k_products<N, R><<<dim3(g.nz, g.np, 2), 3 * FftShape<N>::T, smem, st>>>(s, g);
   }
 }
@@ -1702,8 +1701,7 @@ static void go_products_les_t(const Geom& g, const State& s, cudaStream_t st) {
   using C = typename CplxOf<R>::type;
   const int zr = prod_zr<N>() < g.nz ? prod_zr<N>() : g.nz;
   const size_t smem = (size_t)3 * zr * padded(N) * sizeof(C);
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(k_products_les<N, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (smem > 48 * 1024) smem_limit(k_products_les<N, R>);
   k_products_les<N, R><<<dim3(g.nz / zr, g.np, 2), 3 * FftShape<N>::T * zr, smem, st>>>(s, g, zr);
 }
 template <int N>
@@ -1719,8 +1717,7 @@ static void go_zpass_t(const Geom& g, const Phys& ph, const State& s, int rk, co
   constexpr int T = FftShape<N>::T;
   constexpr bool EFAST = sizeof(R) == sizeof(double);
   size_t smem = (size_t)KT * (3 * padded(N) + 1) * sizeof(typename CplxOf<R>::type);
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(k_zpass_rhs<N, R, EFAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (smem > 48 * 1024) smem_limit(k_zpass_rhs<N, R, EFAST>);
   const dim3 grid = EFAST ? dim3(4, g.kxs / KT, g.np) : dim3(g.kxs / KT, g.np, 4);
   k_zpass_rhs<N, R, EFAST><<<grid, KT * T, smem, st>>>(s, g, ph, rk, ghost);
 }
@@ -1784,7 +1781,6 @@ cudaError_t launch_zpass_spec(const Geom& g, const State& s, cudaStream_t st) {
 // two thirds of the SMs a CTA (64x65x64: 11 with 8 modes, 21 with 32).  It
 // depends on the channel only, so a member of an ensemble gives the bits of
 // its solo run.
-constexpr size_t SMEM_CTA = 227 * 1024;
 constexpr long long CH_MODES = 36000, CH_CTAS = 96;
 static int cn_form(const Geom& g) {
   if (g.sp > CH_MODES) return 0;
@@ -1799,7 +1795,7 @@ template <int M, int CHN, bool SPLITZ, bool B>
 static cudaError_t go_cn_solve_t(const Geom& g, const Phys& ph, const State& s, int rk, const FieldSet& nl,
                                  const MemberArgs* tab, int n, cudaStream_t st) {
   const size_t smem = cn_smem<M, CHN>(g.np);
-  const cudaError_t e = cudaFuncSetAttribute(k_cn_solve<M, CHN, SPLITZ, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = smem_limit(k_cn_solve<M, CHN, SPLITZ, B>);
   if (e) return e;
   k_cn_solve<M, CHN, SPLITZ, B><<<dim3((unsigned)((g.sp + M - 1) / M), n), CHN * M, smem, st>>>(s, g, ph, rk, nl, tab);
   return cudaGetLastError();
@@ -1832,7 +1828,7 @@ static cudaError_t go_tri_coef(const Geom& g, const Phys& ph, TriRow* tri, CnRow
                                int n, cudaStream_t st) {
   const size_t smem = (size_t)g.np * sizeof(double2);
   if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(k_tri_lu<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = smem_limit(k_tri_lu<B>);
     if (e) return e;
   }
   k_tri_rows<B><<<dim3(4, n), 256, 0, st>>>(g, ph, tri, cnr, sc, rk, tab);
@@ -1857,7 +1853,7 @@ template <int M, int CHN, bool B>
 static cudaError_t go_rem_div_t(const Geom& g, const State& s, int rk, int update_cp, const MemberArgs* tab, int n,
                                 cudaStream_t st) {
   const size_t smem = rem_div_smem<M, CHN>(g.np);
-  const cudaError_t e = cudaFuncSetAttribute(k_rem_div_ch<M, CHN, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = smem_limit(k_rem_div_ch<M, CHN, B>);
   if (e) return e;
   k_rem_div_ch<M, CHN, B><<<dim3((unsigned)((g.sp + M - 1) / M), n), CHN * M, smem, st>>>(s, g, rk, update_cp, tab);
   return cudaGetLastError();
@@ -1937,8 +1933,7 @@ static cudaError_t go_products_bt(const Geom& g, const Batch& bt, cudaStream_t s
     constexpr int PROD_SLOTS = prod_slots<R>();
     const size_t smem = (size_t)PROD_SLOTS * 4 * zr * N * sizeof(R) + (size_t)3 * zr * prod_sq<N>() * sizeof(C) +
                         PROD_SLOTS * sizeof(uint64_t);
-    if (smem > 48 * 1024)
-      cudaFuncSetAttribute(k_products_st<N, R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) smem_limit(k_products_st<N, R, true>);
     const int nzb = g.nz / zr;
     const long long res = (long long)(PROD_SLOTS == 4 ? 2 : 3) * sm_count();
     int best = 1;
