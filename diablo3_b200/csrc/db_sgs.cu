@@ -50,16 +50,19 @@ extern "C" int db_sgs_create(void* stream, db_sgs_net** out) {
     db_sgs_destroy(n);
     return DB_ERR_CUDA;
   }
-  cudaMemset(n->params, 0, P);
-  cudaMemset(n->grads, 0, P);
-  cudaMemset(n->m1, 0, P);
-  cudaMemset(n->m2, 0, P);
-  cudaMemset(n->norm, 0, 64 * sizeof(float));
-  cudaMemset(n->err, 0, sizeof(int));
-  {
-    float r[32];
-    for (int f = 0; f < 16; ++f) { r[f] = -3.0e38f; r[16 + f] = 3.0e38f; }   // no fallback until set
-    cudaMemcpy(n->range, r, sizeof(r), cudaMemcpyHostToDevice);
+  float r[32];
+  for (int f = 0; f < 16; ++f) { r[f] = -3.0e38f; r[16 + f] = 3.0e38f; }   // no fallback until set
+  // on the network's stream and waited for: the legacy stream is not ordered
+  // with a caller's non-blocking stream, on which db_sgs_set and
+  // db_sgs_set_range write the same buffers next
+  if (cudaMemsetAsync(n->params, 0, P, n->st) != cudaSuccess || cudaMemsetAsync(n->grads, 0, P, n->st) != cudaSuccess ||
+      cudaMemsetAsync(n->m1, 0, P, n->st) != cudaSuccess || cudaMemsetAsync(n->m2, 0, P, n->st) != cudaSuccess ||
+      cudaMemsetAsync(n->norm, 0, 64 * sizeof(float), n->st) != cudaSuccess ||
+      cudaMemsetAsync(n->err, 0, sizeof(int), n->st) != cudaSuccess ||
+      cudaMemcpyAsync(n->range, r, sizeof(r), cudaMemcpyHostToDevice, n->st) != cudaSuccess ||
+      cudaStreamSynchronize(n->st) != cudaSuccess) {
+    db_sgs_destroy(n);
+    return DB_ERR_CUDA;
   }
   *out = n;
   return DB_OK;
