@@ -1651,9 +1651,10 @@ extern "C" int db_sgs_targets(db_ctx* c, int fx, int fy, int fz, const double* g
   for (int j = 1; j <= nyc + 1; ++j) c2dy[j] = 2.0 * (cgyf[j] - cgyf[j - 1]);
   double* d_dy = nullptr;
   CK(cudaMalloc(&d_dy, c2dy.size() * sizeof(double)));
-  CK(cudaMemcpy(d_dy, c2dy.data(), c2dy.size() * sizeof(double), cudaMemcpyHostToDevice));
   State& s = c->s;
   cudaStream_t st = c->st;
+  // on the stream whose kernels read it (the legacy stream is not ordered with it)
+  CK(cudaMemcpyAsync(d_dy, c2dy.data(), c2dy.size() * sizeof(double), cudaMemcpyHostToDevice, st));
   // the state and its x and z derivatives in physical space (no ghost overlay)
   CK(launch_inv_z(g, fset(s.cu1, s.cu2, s.cu3, s.cth, s.cu1, s.cu2, s.cu3, s.cth),
                   fset(s.xh[0], s.xh[1], s.xh[2], s.xh[3], s.xh[4], s.xh[5], s.xh[6], s.xh[7]), 8, st, 0xF0u));

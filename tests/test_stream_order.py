@@ -24,7 +24,7 @@ def program(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("what", ["init", "init mixed", "sgs"])
+@pytest.mark.parametrize("what", ["init", "init mixed", "sgs", "targets"])
 def test_no_two_streams_on_one_buffer(program, what):
     r = subprocess.run([program, what], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout
