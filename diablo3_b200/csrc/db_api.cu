@@ -867,6 +867,7 @@ static cudaError_t substep(db_ctx* c, int rk /* 0-based */, bool les) {
   if ((e = cudaEventRecord(c->ev_fork, st))) return e;
   if ((e = cudaStreamWaitEvent(c->st_side, c->ev_fork, 0))) return e;
   if ((e = launch_tri_coef(g, c->ph, s, rk, c->st_side))) return e;
+  n += 2;
   if ((e = cudaEventRecord(c->ev_join, c->st_side))) return e;
   if (les) {
     // les_chan / les_chan_th: ghost rows, then the state and its x and z
@@ -889,16 +890,18 @@ static cudaError_t substep(db_ctx* c, int rk /* 0-based */, bool les) {
     } else {
       if ((e = launch_les_amd(g, c->ph, s, st))) return e;
     }
-    n += 2;
+    n += 4;
   } else {
     // velocity and buoyancy to physical space (solver.f90:635-643)
     if ((e = launch_inv_z(g, fset(s.cu1, s.cu2, s.cu3, s.cth), fset(s.xh[0], s.xh[1], s.xh[2], s.xh[3]), 4, st))) return e;
     mark(c, rk, 1);
     if ((e = launch_inv_x(g, fset(s.xh[0], s.xh[1], s.xh[2], s.xh[3]), fset(s.u1, s.u2, s.u3, s.th), 4, st))) return e;
     mark(c, rk, 2);
+    n += 2;
   }
   // nonlinear products (+ SGS forcing) + x-FFT
   if ((e = launch_products(g, s, st, les))) return e;
+  n += 1;
   mark(c, rk, 3);
   const bool cfl_step = rk == 2 && c->p.variable_dt;
   if (spectral) {
@@ -911,7 +914,7 @@ static cudaError_t substep(db_ctx* c, int rk /* 0-based */, bool les) {
     if ((e = cudaStreamWaitEvent(st, c->ev_join, 0))) return e;
     if ((e = launch_rhs_cn(g, c->ph, s, rk, st))) return e;
     mark(c, rk, 6);
-    n += 5;
+    n += 1 + rhs_cn_kernels(g);
     // CFL on the last substep from the new velocity before the projection
     // (solver.f90:1241-1244): u1..u3 to physical space for it
     if (cfl_step) {
@@ -937,7 +940,7 @@ static cudaError_t substep(db_ctx* c, int rk /* 0-based */, bool les) {
     // reads it
     if ((e = launch_thomas_les(g, s, rk, st, cfl_step))) return e;
     mark(c, rk, 6);
-    n += 7;
+    n += (g.prec ? 1 : 3) + 2;   // the z-pass in one kernel or in three stages
     // CFL on the last substep (solver.f90:1241-1244)
     if (cfl_step) {
       CflCtl ctl{c->p.cfl, c->p.time_limit, c->p.variable_dt, c->p.update_dt, 0};
@@ -968,15 +971,16 @@ static cudaError_t substep(db_ctx* c, int rk /* 0-based */, bool les) {
       if ((e = launch_fwd_z(g, fset(s.xh[0], s.xh[1], s.xh[2], s.xh[3]), fset(s.cu1, s.cu2, s.cu3, s.cth), 4, st, 0,
                             ov))) return e;
     }
+    n += 2;
   }
   mark(c, rk, 9);
   if ((e = launch_rem_div(g, s, rk, 1, st))) return e;
+  n += 1;
   if (rk == 2 && c->p.variable_dt) {
     if ((e = launch_apply_dt(s.sc, st))) return e;
     n += 1;
   }
   mark(c, rk, 10);
-  n += 3;
   c->launches += n;
   return cudaSuccess;
 }

@@ -246,6 +246,7 @@ cudaError_t launch_tri_coef(const Geom& g, const Phys& ph, const State& s, int r
 // in spectral space (k_rhs_cn, k_cn_back or k_cn_solve), the state in place
 cudaError_t launch_zpass_spec(const Geom& g, const State& s, cudaStream_t st);
 cudaError_t launch_rhs_cn(const Geom& g, const Phys& ph, const State& s, int rk, cudaStream_t st);
+int rhs_cn_kernels(const Geom& g);   // the kernels it launches
 
 struct CflCtl {
   double cfl, time_limit;

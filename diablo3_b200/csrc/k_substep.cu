@@ -1818,7 +1818,8 @@ static cudaError_t go_cn_solve(const Geom& g, const Phys& ph, const State& s, in
                                const MemberArgs* tab, int n, cudaStream_t st) {
   return g.prec ? go_cn<false, B>(g, ph, s, rk, nl, tab, n, st) : go_cn<true, B>(g, ph, s, rk, nl, tab, n, st);
 }
-int substep_batch_kernels(const Geom& g) { return cn_form(g) ? 8 : 9; }
+int rhs_cn_kernels(const Geom& g) { return cn_form(g) ? 1 : 2; }
+int substep_batch_kernels(const Geom& g) { return 7 + rhs_cn_kernels(g); }
 cudaError_t launch_rhs_cn(const Geom& g, const Phys& ph, const State& s, int rk, cudaStream_t st) {
   const FieldSet nl = fset(s.crs[0], s.crs[1], s.crs[2], s.crs[3], s.nls[4], s.nls[5], s.nls[6], s.nls[7]);
   return go_cn_solve<false>(g, ph, s, rk, nl, nullptr, 1, st);
