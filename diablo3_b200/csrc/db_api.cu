@@ -793,8 +793,15 @@ extern "C" int db_fft_xz_to_physical(db_ctx* c, double* buf) {
 // device-resident forms: the same transforms on a device array in the
 // reference layout, every layout change on the device, stream-ordered on
 // the context's stream (no host synchronisation)
-extern "C" int db_fft_xz_to_fourier_dev(db_ctx* c, double* d) {
+static int check_dev_array(db_ctx* c, const double* d) {
   if (!c || !d) return DB_ERR_ARG;
+  // bulk copies and 16-byte accesses: anything else would fault on the device
+  if (reinterpret_cast<uintptr_t>(d) % 16) return fail(c, DB_ERR_ARG, "the device array must be 16-byte aligned");
+  return DB_OK;
+}
+
+extern "C" int db_fft_xz_to_fourier_dev(db_ctx* c, double* d) {
+  if (int rc = check_dev_array(c, d)) return rc;
   const Geom& g = c->g;
   CK(launch_fwd_x_ref(g, d, c->s.xh[0], c->st));
   CK(launch_fwd_z(g, fset(c->s.xh[0]), fset(c->s.phi_g), 1, c->st));
@@ -804,7 +811,7 @@ extern "C" int db_fft_xz_to_fourier_dev(db_ctx* c, double* d) {
 }
 
 extern "C" int db_fft_xz_to_physical_dev(db_ctx* c, double* d) {
-  if (!c || !d) return DB_ERR_ARG;
+  if (int rc = check_dev_array(c, d)) return rc;
   const Geom& g = c->g;
   CK(launch_ref_to_spec(g, c->p.nx, c->p.nz, reinterpret_cast<const double2*>(d), c->s.phi_g, c->st));
   CK(launch_inv_z(g, fset(c->s.phi_g), fset(c->s.xh[0]), 1, c->st));

@@ -164,8 +164,10 @@ int db_fft_xz_to_physical(db_ctx* ctx, double* inout);
 /* The same two transforms on a DEVICE array in the reference layout (for
  * callers whose fields already live in device memory), in place, with every
  * layout change on the device.  Stream-ordered on the context's stream: the
- * call returns once the work is enqueued.  The physical layout's padding
- * (x >= Nx, z >= Nz) is neither read nor written, as in the host forms. */
+ * call returns once the work is enqueued.  The array must be 16-byte aligned
+ * (DB_ERR_ARG otherwise).  The values of the physical layout's padding
+ * (x >= Nx, z >= Nz) are not used and the padding is not written by
+ * fft_xz_to_physical, as in the host forms. */
 int db_fft_xz_to_fourier_dev(db_ctx* ctx, double* d_inout);
 int db_fft_xz_to_physical_dev(db_ctx* ctx, double* d_inout);
 

@@ -48,3 +48,18 @@ def test_device_transforms_match_host_forms(prec):
     tol = 1e-12 if prec == 0 else 1e-5
     assert np.abs(again - spec_host).max() <= tol * np.abs(spec_host).max()
     ch.close()
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+def test_misaligned_device_array_is_refused(prec):
+    """A float64 view 8 bytes off: an error code from both calls, nothing launched."""
+    from diablo3_b200.channel import Channel
+    from diablo3_b200.lib import DiabloError
+    p = config0_params(nx=16, ny=9, nz=16, precision=prec)
+    with Channel(p, grid_for(p)) as ch:
+        d = torch.ones(ch.new_real().size + 1, dtype=torch.float64, device="cuda")
+        for call in (ch.fft_xz_to_fourier_dev, ch.fft_xz_to_physical_dev):
+            with pytest.raises(DiabloError, match="aligned"):
+                call(d[1:])
+        torch.cuda.synchronize()
+        assert bool((d == 1.0).all())
