@@ -32,6 +32,22 @@ namespace db {
 // 1.32 -> 1.44 ms, and keeps one plane per CTA)
 constexpr int ZPJ = 2;
 
+// Between two planes of such a CTA: the exchange buffers are free again, and
+// every store of the plane before has left its registers.  The fence is for
+// the latter: nvcc 12.9.86 (-O2, -O3) let a plane's last store go out with
+// registers that already held the next plane's addresses.  A warp's row of an
+// even plane came out wrong in 0.2 to 7 % of the FP32 forward transforms of
+// 128x63x64 and 256x33x64, and in one arrangement of the loop a store went to a
+// wrong address (illegal memory access).  With the fence, or with the planes
+// as straight-line code, none in 77000 transforms each, at the same time.
+// us a substep, 512x257x512: k_fwd_z, straight-line, 1402 (1545 rolled, without
+// the fence); k_inv_z FP64, rolled, 775 (731; straight-line it spills, 802),
+// FP32, straight-line, 680 (653; rolled 716).
+__device__ __forceinline__ void next_plane() {
+  __threadfence_block();
+  __syncthreads();
+}
+
 // a hint that brings the line holding p into L2 (p must be a valid global
 // address)
 __device__ __forceinline__ void prefetch_l2(const void* p) {
@@ -154,10 +170,11 @@ __global__ void __launch_bounds__(256, DB_LB_FFT) k_fwd_z(const __grid_constant_
   C* sq = sm + seq * (padded(N) + 1);   // staggered so the ns columns use different banks
   const C* twt = tw_z<R>(g);   // twiddles fetched per pass (fewer live registers)
   const double s = 1.0 / (double)N;
+#pragma unroll
   for (int jj = 0; jj < ZPJ; ++jj) {
     const int j = blockIdx.y * ZPJ + jj;
     if (j >= g.np) break;                 // uniform over the CTA
-    if (jj > 0) __syncthreads();          // the exchange buffers are free again
+    if (jj > 0) next_plane();
     const C* src = (const C*)in.p[f] + (long long)j * g.hp + kx;
     if (active && jj + 1 < ZPJ && j + 1 < g.np) {
 #pragma unroll
@@ -291,10 +308,9 @@ __global__ void __launch_bounds__(256, DB_LB_FFT) k_inv_z(const __grid_constant_
   const bool dz = (dmask >> f) & 1u;
   // ZPJ planes in turn, as k_fwd_z (the next plane's retained rows
   // prefetched into L2)
+#pragma unroll (sizeof(R) == sizeof(float) ? ZPJ : 1)
   for (int jj = 0; jj < ZPJ; ++jj) {
     const int j = blockIdx.y * ZPJ + jj;
-    if (j >= g.np) break;                 // uniform over the CTA
-    if (jj > 0) __syncthreads();          // the exchange buffers are free again
     const double2* src = (const double2*)in.p[f] + (long long)j * g.sp + kx;
     if (active && jj + 1 < ZPJ && j + 1 < g.np) {
 #pragma unroll
@@ -327,6 +343,8 @@ __global__ void __launch_bounds__(256, DB_LB_FFT) k_inv_z(const __grid_constant_
 #pragma unroll
       for (int q = 0; q < E; ++q) dst[(long long)(lane + q * T) * g.kxs] = v[q];
     }
+    if (jj + 1 == ZPJ || j + 1 >= g.np) break;   // uniform over the CTA
+    next_plane();
   }
 }
 
