@@ -925,7 +925,7 @@ __device__ __forceinline__ double2 cn_rhs(const CnRow& row, const CnMode& k, con
   return w;
 }
 
-// Two forms (cn_form): k_rhs_cn and k_cn_back walk all planes with one thread
+// Two forms (cn_chunks): k_rhs_cn and k_cn_back walk all planes with one thread
 // per mode (many modes), k_cn_solve splits the planes into chunks.
 //
 // k_rhs_cn: one thread per retained mode walks the planes upward and runs
@@ -1770,27 +1770,43 @@ cudaError_t launch_zpass_spec(const Geom& g, const State& s, cudaStream_t st) {
   return launch_fwd_z_nl(g, fset(s.xh[0], s.xh[1], s.xh[2], s.xh[3], s.xh[4], s.xh[5], s.xh[6], s.xh[7]),
                          fset(s.crs[0], s.crs[1], s.crs[2], s.crs[3]), st);
 }
-// Modes per CTA of k_cn_solve (0: k_rhs_cn and k_cn_back).  One thread per
-// mode needs tens of thousands of modes to hide its chain of loads; the chunked
-// form has 4 to 32 times the threads.  Two-kernel -> chunked, us a substep:
-// 64x65x64 261 -> 11, 256x129x256 666 -> 237, 512x129x256 756 -> 444, 32
-// channels of 128x65x128 (mixed) 947 -> 844, but 512x257x512 2050 -> 2200, so
-// planes of more than 36000 modes keep the two kernels.  Wide CTAs read longer
-// rows and scan less (32 channels: 1363 with 8 modes, 999 with 16, 844 with
-// 32), so the widest one whose columns fit shared memory and that still gives
-// two thirds of the SMs a CTA (64x65x64: 11 with 8 modes, 21 with 32).  It
-// depends on the channel only, so a member of an ensemble gives the bits of
-// its solo run.
-constexpr long long CH_MODES = 36000, CH_CTAS = 96;
-static int cn_form(const Geom& g) {
-  if (g.sp > CH_MODES) return 0;
-  if (cn_smem<32, 8>(g.np) <= SMEM_CTA && g.sp >= 32 * CH_CTAS) return 32;
-  if (cn_smem<16, 16>(g.np) <= SMEM_CTA && g.sp >= 16 * CH_CTAS) return 16;
-  if (cn_smem<8, 32>(g.np) <= SMEM_CTA) return 8;
-  if (cn_smem<4, 32>(g.np) <= SMEM_CTA) return 4;
-  return 0;
+// Chunks of a column of `rows` rows: 32, halved until a chunk has `least32`
+// rows, then (fewer chunks) `least`.
+static int chunks_for(int rows, long long least32, long long least) {
+  int c = 32;
+  if ((rows + c - 1) / c < least32) c = 16;
+  while (c < 32 && c > 4 && (rows + c - 1) / c < least) c >>= 1;
+  return c;
 }
-static int cn_chunks(const Geom& g) { return cn_form(g) == 32 ? 8 : (cn_form(g) == 16 ? 16 : 32); }
+// Chunks of k_cn_solve's columns (0: k_rhs_cn and k_cn_back).  It depends on
+// the channel only, so a member of an ensemble gives the bits of its solo run;
+// what is best for one channel and for a batch of them lies apart:
+//  - One channel: more chunks, shorter chains (64x65x64, us a substep: 13 with
+//    32 chunks, 17 with 16, 25 with 8, 158 with one thread per mode).
+//  - 32 channels: every thread's fixed cost and the scans count, so chunks want
+//    rows: 64x17x128 (mixed) 444 with 32 chunks, 308 with 16, 198 with 8, 141 with
+//    4 (130 with one thread per mode); 64x33x64 325, 209, 157 (198).
+// A chunk has 1 row at least in planes of up to 400 modes, 2 up to 800, 3 up to
+// 1200, 5 from 1600.  A substep of 32 channels (32 to 128 points in x and z, ny 17
+// to 129) then takes 0.4 to 1.002 of its time with one thread per mode, where it
+// took up to 1.34; of one channel it costs 1 to 5 us.  Planes from 1536 modes
+// take at most 16 chunks, from 3072 at most 8 (wider CTAs read longer rows: 32
+// channels of 128x65x128 1447 with 8 modes a CTA, 1053 with 16, 878 with 32).
+// Planes of more than 36000 modes keep the two kernels (512x257x512 1664 in
+// FP64 and 1345 mixed; the chunked form was 2200); between 30052 and 58652
+// modes there are none.  At 29412 modes the two kernels are about as fast:
+// 512x129x256 434 (FP64) and 464 (mixed) against 444 and 408 chunked, but
+// 512x257x256, whose columns leave 8 modes a CTA, 850 and 910 against 1123 and
+// 949.
+constexpr long long CH_MODES = 36000, CH_CTAS = 96;
+static int cn_chunks(const Geom& g) {
+  if (g.sp > CH_MODES) return 0;
+  const long long least = min(5LL, 1 + g.sp / 400);
+  int c = chunks_for(g.np, least, least);
+  if (g.sp >= 32 * CH_CTAS && cn_smem<32, 8>(g.np) <= SMEM_CTA) c = min(c, 8);
+  else if (g.sp >= 16 * CH_CTAS && cn_smem<16, 16>(g.np) <= SMEM_CTA) c = min(c, 16);
+  return c == 32 && cn_smem<4, 32>(g.np) > SMEM_CTA ? 0 : c;
+}
 template <int M, int CHN, bool SPLITZ, bool B>
 static cudaError_t go_cn_solve_t(const Geom& g, const Phys& ph, const State& s, int rk, const FieldSet& nl,
                                  const MemberArgs* tab, int n, cudaStream_t st) {
@@ -1803,11 +1819,13 @@ static cudaError_t go_cn_solve_t(const Geom& g, const Phys& ph, const State& s, 
 template <bool SPLITZ, bool B>
 static cudaError_t go_cn(const Geom& g, const Phys& ph, const State& s, int rk, const FieldSet& nl,
                          const MemberArgs* tab, int n, cudaStream_t st) {
-  switch (cn_form(g)) {
-    case 32: return go_cn_solve_t<32, 8, SPLITZ, B>(g, ph, s, rk, nl, tab, n, st);
+  switch (cn_chunks(g)) {
+    case 4: return go_cn_solve_t<32, 4, SPLITZ, B>(g, ph, s, rk, nl, tab, n, st);
+    case 8: return go_cn_solve_t<32, 8, SPLITZ, B>(g, ph, s, rk, nl, tab, n, st);
     case 16: return go_cn_solve_t<16, 16, SPLITZ, B>(g, ph, s, rk, nl, tab, n, st);
-    case 8: return go_cn_solve_t<8, 32, SPLITZ, B>(g, ph, s, rk, nl, tab, n, st);
-    case 4: return go_cn_solve_t<4, 32, SPLITZ, B>(g, ph, s, rk, nl, tab, n, st);
+    case 32:
+      if (cn_smem<8, 32>(g.np) <= SMEM_CTA) return go_cn_solve_t<8, 32, SPLITZ, B>(g, ph, s, rk, nl, tab, n, st);
+      return go_cn_solve_t<4, 32, SPLITZ, B>(g, ph, s, rk, nl, tab, n, st);
   }
   k_rhs_cn<SPLITZ, B><<<dim3((unsigned)((g.sp + 31) / 32), n), 32, 0, st>>>(s, g, ph, rk, nl, tab);
   k_cn_back<B><<<dim3((unsigned)((2 * g.sp + 127) / 128), 4, n), 128, 0, st>>>(s, g, nl, tab);
@@ -1818,7 +1836,7 @@ static cudaError_t go_cn_solve(const Geom& g, const Phys& ph, const State& s, in
                                const MemberArgs* tab, int n, cudaStream_t st) {
   return g.prec ? go_cn<false, B>(g, ph, s, rk, nl, tab, n, st) : go_cn<true, B>(g, ph, s, rk, nl, tab, n, st);
 }
-int rhs_cn_kernels(const Geom& g) { return cn_form(g) ? 1 : 2; }
+int rhs_cn_kernels(const Geom& g) { return cn_chunks(g) ? 1 : 2; }
 int substep_batch_kernels(const Geom& g) { return 7 + rhs_cn_kernels(g); }
 cudaError_t launch_rhs_cn(const Geom& g, const Phys& ph, const State& s, int rk, cudaStream_t st) {
   const FieldSet nl = fset(s.crs[0], s.crs[1], s.crs[2], s.crs[3], s.nls[4], s.nls[5], s.nls[6], s.nls[7]);
@@ -1833,7 +1851,7 @@ static cudaError_t go_tri_coef(const Geom& g, const Phys& ph, TriRow* tri, CnRow
     if (e) return e;
   }
   k_tri_rows<B><<<dim3(4, n), 256, 0, st>>>(g, ph, tri, cnr, sc, rk, tab);
-  k_tri_lu<B><<<dim3(4, n), 256, smem, st>>>(g.np, cn_chunks(g), tri, cnr, tab);
+  k_tri_lu<B><<<dim3(4, n), 256, smem, st>>>(g.np, max(1, cn_chunks(g)), tri, cnr, tab);
   return cudaGetLastError();
 }
 cudaError_t launch_tri_coef(const Geom& g, const Phys& ph, const State& s, int rk, cudaStream_t st) {
@@ -1862,12 +1880,15 @@ static cudaError_t go_rem_div_t(const Geom& g, const State& s, int rk, int updat
 template <bool B>
 static cudaError_t go_rem_div(const Geom& g, const State& s, int rk, int update_cp, const MemberArgs* tab, int n,
                               cudaStream_t st) {
-  // as cn_form; us a substep: 64x65x64 59 -> 6, 256x129x256 165 -> 91, 32
-  // channels of 128x65x128 329 -> 338 (wide CTAs; 517 with 8 modes) but alone
-  // 66 -> 23, 512x257x512 590 -> 785 (stays)
+  // as cn_chunks, 8 to 32 chunks.  us a substep, one channel 64x65x64 8 with 32
+  // chunks, 8 with 16, 16 with 8 (61 with one thread per column); 32 channels
+  // 64x65x128 279, 201, 180 (225), 64x33x64 85, 65, 56 (87), 128x65x128 529, 367,
+  // 337 (352).  512x257x512 590 against 785 chunked (stays).
   if (g.sp <= CH_MODES) {
-    if (rem_div_smem<32, 8>(g.np) <= 75 * 1024 && g.sp >= 32 * CH_CTAS)   // three CTAs an SM
+    const int c = chunks_for(g.ny, min(5LL, 1 + g.sp / 300), min(5LL, 1 + g.sp / 400));
+    if (c <= 8 || (rem_div_smem<32, 8>(g.np) <= 75 * 1024 && g.sp >= 32 * CH_CTAS))   // three CTAs an SM
       return go_rem_div_t<32, 8, B>(g, s, rk, update_cp, tab, n, st);
+    if (c == 16) return go_rem_div_t<16, 16, B>(g, s, rk, update_cp, tab, n, st);
     if (rem_div_smem<8, 32>(g.np) <= SMEM_CTA) return go_rem_div_t<8, 32, B>(g, s, rk, update_cp, tab, n, st);
   }
   const dim3 grid((2 * (g.nkx + 1) + 127) / 128, g.nkzp, n);
