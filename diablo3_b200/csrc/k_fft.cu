@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(256, DB_LB_FFT) k_inv_x(const __grid_constant_
 // accumulate: out = base + transform, base = out itself, or for rows 0, 1,
 // Nyp, Nyp+1 the ghost overlay (field f % 4) when one is given
 // B: member-batched (blockIdx.z = member * nf + field)
-template <int N, typename R, bool ACC, bool B = false>
+template <int N, typename R, bool ACC, bool B = false, int PJ = ZPJ>
 __global__ void __launch_bounds__(256, DB_LB_FFT) k_fwd_z(const __grid_constant__ FieldSet in0, const __grid_constant__ FieldSet out0, Geom g0, int accumulate,
                                                           const double2* __restrict__ ghost, const __grid_constant__ Batch bt) {
   const int m = B ? (int)blockIdx.z / bt.nf : 0, f = B ? (int)blockIdx.z - m * bt.nf : (int)blockIdx.z;
@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(256, DB_LB_FFT) k_fwd_z(const __grid_constant_
   constexpr int E = S::E, T = S::T;
   // column-fastest mapping: a warp reads ns consecutive kx of 32/ns rows
   // (whole sectors); the sequence's threads are then spread over the CTA
-  // and the exchanges use CTA barriers.  A CTA transforms ZPJ planes in
+  // and the exchanges use CTA barriers.  A CTA transforms PJ planes in
   // turn, the next plane's tile prefetched into L2 while this one is
   // transformed.
   const int ns = blockDim.x / T;
@@ -171,12 +171,12 @@ __global__ void __launch_bounds__(256, DB_LB_FFT) k_fwd_z(const __grid_constant_
   const C* twt = tw_z<R>(g);   // twiddles fetched per pass (fewer live registers)
   const double s = 1.0 / (double)N;
 #pragma unroll
-  for (int jj = 0; jj < ZPJ; ++jj) {
-    const int j = blockIdx.y * ZPJ + jj;
+  for (int jj = 0; jj < PJ; ++jj) {
+    const int j = blockIdx.y * PJ + jj;
     if (j >= g.np) break;                 // uniform over the CTA
     if (jj > 0) next_plane();
     const C* src = (const C*)in.p[f] + (long long)j * g.hp + kx;
-    if (active && jj + 1 < ZPJ && j + 1 < g.np) {
+    if (active && jj + 1 < PJ && j + 1 < g.np) {
 #pragma unroll
       for (int q = 0; q < E; ++q) prefetch_l2(src + g.hp + (long long)(lane + q * T) * g.kxs);
     }
@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(znl_threads<N>(), FftShape<N>::T >= 256 ? 1 : 
 // and its FP32 rounding scales with the fluctuation (the consumers add the
 // mean back)
 // B: member-batched (blockIdx.z = member * nf + field; no dmask, ghost or mean)
-template <int N, typename R, bool B = false>
+template <int N, typename R, bool B = false, int PJ = ZPJ>
 __global__ void __launch_bounds__(256, DB_LB_FFT) k_inv_z(const __grid_constant__ FieldSet in0, const __grid_constant__ FieldSet out0, Geom g0, unsigned dmask,
                                                           const double2* __restrict__ ghost, double* __restrict__ mean,
                                                           const __grid_constant__ Batch bt) {
@@ -306,13 +306,13 @@ __global__ void __launch_bounds__(256, DB_LB_FFT) k_inv_z(const __grid_constant_
   C* sq = sm + seq * (padded(N) + 1);
   const C* twt = tw_z<R>(g);   // twiddles fetched per pass (fewer live registers)
   const bool dz = (dmask >> f) & 1u;
-  // ZPJ planes in turn, as k_fwd_z (the next plane's retained rows
+  // PJ planes in turn, as k_fwd_z (the next plane's retained rows
   // prefetched into L2)
-#pragma unroll (sizeof(R) == sizeof(float) ? ZPJ : 1)
-  for (int jj = 0; jj < ZPJ; ++jj) {
-    const int j = blockIdx.y * ZPJ + jj;
+#pragma unroll (sizeof(R) == sizeof(float) ? PJ : 1)
+  for (int jj = 0; jj < PJ; ++jj) {
+    const int j = blockIdx.y * PJ + jj;
     const double2* src = (const double2*)in.p[f] + (long long)j * g.sp + kx;
-    if (active && jj + 1 < ZPJ && j + 1 < g.np) {
+    if (active && jj + 1 < PJ && j + 1 < g.np) {
 #pragma unroll
       for (int q = 0; q < E; ++q) {
         const int z = lane + q * T;
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(256, DB_LB_FFT) k_inv_z(const __grid_constant_
 #pragma unroll
       for (int q = 0; q < E; ++q) dst[(long long)(lane + q * T) * g.kxs] = v[q];
     }
-    if (jj + 1 == ZPJ || j + 1 >= g.np) break;   // uniform over the CTA
+    if (jj + 1 == PJ || j + 1 >= g.np) break;   // uniform over the CTA
     next_plane();
   }
 }
@@ -646,6 +646,13 @@ int sm_count() {
   return n;
 }
 
+// one plane per CTA in the z-passes: where two would leave an SM without its
+// three CTAs, and the second plane only waits for the first (us a pass with two
+// and with one: inverse of 4 fields 64x65x64 FP64 6.5, 4.5, mixed 6.7, 4.4;
+// 64x33x256 mixed 11.2, 8.0; 128x65x128 FP64 17.3, 17.9, mixed 15.6, 14.4; forward
+// of one field 64x33x256 FP32 7.0, 4.8)
+static bool plane_each(const dim3& two) { return (long long)two.x * two.y * two.z < 3LL * sm_count(); }
+
 template <int N, typename R, bool REF = false>
 static void go_fwd_x_t(const Geom& g, FieldSet in, FieldSet out, int nf, cudaStream_t st) {
   using C = typename CplxOf<R>::type;
@@ -691,10 +698,13 @@ static void go_fwd_z_t(const Geom& g, FieldSet in, FieldSet out, int nf, int acc
   using C = typename CplxOf<R>::type;
   const int ns = zpass_ns<N>(g);
   size_t smem = (size_t)ns * (padded(N) + 1) * sizeof(C);
-  const dim3 grid((g.kxs + ns - 1) / ns, (g.np + ZPJ - 1) / ZPJ, nf);
+  const dim3 grid((g.kxs + ns - 1) / ns, (g.np + ZPJ - 1) / ZPJ, nf), one(grid.x, g.np, nf);
   if (acc) {
     smem_attr(k_fwd_z<N, R, true>, smem);
     k_fwd_z<N, R, true><<<grid, ns * FftShape<N>::T, smem, st>>>(in, out, g, 1, ghost, Batch{});
+  } else if (plane_each(grid)) {
+    smem_attr(k_fwd_z<N, R, false, false, 1>, smem);
+    k_fwd_z<N, R, false, false, 1><<<one, ns * FftShape<N>::T, smem, st>>>(in, out, g, 0, ghost, Batch{});
   } else {
     smem_attr(k_fwd_z<N, R, false>, smem);
     k_fwd_z<N, R, false><<<grid, ns * FftShape<N>::T, smem, st>>>(in, out, g, 0, ghost, Batch{});
@@ -706,9 +716,14 @@ static void go_inv_z_t(const Geom& g, FieldSet in, FieldSet out, int nf, unsigne
   using C = typename CplxOf<R>::type;
   const int ns = zpass_ns<N>(g);
   size_t smem = (size_t)ns * (padded(N) + 1) * sizeof(C);
-  smem_attr(k_inv_z<N, R>, smem);
-  k_inv_z<N, R><<<dim3((g.kxs + ns - 1) / ns, (g.np + ZPJ - 1) / ZPJ, nf), ns * FftShape<N>::T, smem, st>>>(in, out, g, dmask, ghost,
-                                                                                          mean, Batch{});
+  const dim3 grid((g.kxs + ns - 1) / ns, (g.np + ZPJ - 1) / ZPJ, nf), one(grid.x, g.np, nf);
+  if (plane_each(grid)) {
+    smem_attr(k_inv_z<N, R, false, 1>, smem);
+    k_inv_z<N, R, false, 1><<<one, ns * FftShape<N>::T, smem, st>>>(in, out, g, dmask, ghost, mean, Batch{});
+  } else {
+    smem_attr(k_inv_z<N, R>, smem);
+    k_inv_z<N, R><<<grid, ns * FftShape<N>::T, smem, st>>>(in, out, g, dmask, ghost, mean, Batch{});
+  }
 }
 template <int N, typename R>
 static void go_fwd_z_nl_t(const Geom& g, FieldSet in, FieldSet out, cudaStream_t st) {

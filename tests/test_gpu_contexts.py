@@ -84,3 +84,22 @@ def test_channels_of_two_sizes_on_two_threads(sizes):
     assert same([channel_state(ch, p) for p, ch in pairs], want)
     for _, ch in pairs:
         ch.close()
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("n", [(128, 63, 64), (64, 33, 128)])
+def test_equal_members_stay_equal(n, prec):
+    """24 members with one state: 60 steps later every bit is still the same in all of them."""
+    from diablo3_b200.ensemble import Ensemble
+    p = config0_params(nx=n[0], ny=n[1], nz=n[2], precision=prec)
+    ens = Ensemble([p] * 24, grid_for(p), init=False)
+    ens.members[0].init_flow(seed=3)
+    state = ens.members[0].download_state()
+    for m in ens.members:
+        m.upload_state(state)
+    ens.step(60)
+    first = channel_state(ens.members[0], p)
+    for m in ens.members[1:]:
+        s = channel_state(m, p)
+        assert all(np.array_equal(s[f], first[f]) for f in s)
+    ens.close()
