@@ -220,10 +220,10 @@ __global__ void __launch_bounds__(3 * FftShape<N>::T, FftShape<N>::T >= 128 ? 1 
 //        overlapping the second group's FFT and the next plane's first
 //        group.  With an exchange stride of padded(N) - 1 a CTA holds
 //        < 76 KB of shared memory, and three CTAs share an SM.
-// Bound by instructions (IPC 2 of 4, DRAM at 8 to 15 %): with the group and
-// sequence branches out of the element loops, one sequence per warp, and three
-// CTAs of the persistent FP32 grid, us a substep 512x257x512 4129 -> 3735
-// (FP64) and 3614 -> 2678 (FP32), 32 channels of 128x65x128 1494 -> 1227.
+// Bound by instructions (IPC 2 of 4, DRAM at 8 to 15 %).  With the group and
+// sequence branches out of the element loops and one sequence per warp, us a
+// substep: 512x257x512 FP64 4129 -> 3735; FP32, three CTAs of the persistent
+// grid on both sides, 2835 -> 2674 (two CTAs were the default before: 3614).
 template <typename R>
 constexpr int prod_slots() { return sizeof(R) == sizeof(double) ? 4 : 3; }
 constexpr uint32_t PROD_WAIT = 1u << 24;
@@ -897,7 +897,8 @@ __device__ __forceinline__ CnMode cn_mode(const State& s, const Geom& g, const P
 // cp of planes j and j-1, NL n (n + i kz z with SPLITZ) and the old cf h.
 // rhs_eval with the row's metric factors and the mode's products formed once:
 // its divisions and branches were two thirds of the solve's instructions
-// (k_rhs_cn at 512x257x512 1472 -> 1331 us a substep, mixed 1350 -> 1012).
+// (k_rhs_cn at 512x257x512 1472 -> 1331 us a substep, mixed 1350 -> 1012, for
+// 232 and 152 bytes of spills a thread at its 128 registers, 124 before in FP64).
 template <bool SPLITZ>
 __device__ __forceinline__ double2 cn_rhs(const CnRow& row, const CnMode& k, const Phys& ph, int e, const double2* um,
                                           const double2* uc, double2 un, double2 v2, double2 cp, double2 pm, double2 n,
@@ -931,10 +932,9 @@ __device__ __forceinline__ double2 cn_rhs(const CnRow& row, const CnMode& k, con
 // k_rhs_cn: one thread per retained mode walks the planes upward and runs
 // the four equations (z-pass order 0 u1, 1 u3, 2 u2, 3 th) together,
 // joining the spectral RHS with the forward sweep: NL from the z-pass (or
-// its Z(N), Z(M) parts, SPLITZ), cr and cf (stored) by rhs_eval, the
-// explicit CN term from
-// the old state planes j-1..j+1 and y_j = v_j + a'_j y_{j-1}; y_j
-// overwrites NL of plane j.  The planes j-1, j, j+1 of cu1, cu3, cu2, cth
+// its Z(N), Z(M) parts, SPLITZ), cr, cf (stored) and the explicit CN term
+// from the old state planes j-1..j+1 by cn_rhs, and y_j = v_j + a'_j y_{j-1};
+// y_j overwrites NL of plane j.  The planes j-1, j, j+1 of cu1, cu3, cu2, cth
 // (the CN explicit terms and the cross terms of the RHS) and cp of planes
 // j-1, j stay in registers as the walk moves up, so each state plane is
 // loaded once for all four equations (13 loads per plane and mode, 17 with
