@@ -362,8 +362,16 @@ __global__ void __launch_bounds__(192, prod_slots<R>() == 4 ? 2 : 3) k_products_
 // closure's column walk (product + SGS forcing, k_les.cu, les[0..10] in
 // (group, sequence, part) order), so a CTA of zr z rows of one plane and one
 // group loads its pairs, transforms and separates; no neighbouring planes.
+// CTAs an SM holds: three in FP64 (105 registers left two: 512x65x512 902 -> 700
+// us, 128x65x128 57 -> 47), five in FP32 at Nx 128 and 256 (73 left four:
+// 256x129x256 241 -> 223; Nx 512 503 against 510 with five).
 template <int N, typename R>
-__global__ void __launch_bounds__(3 * FftShape<N>::T * prod_zr<N>()) k_products_les(const __grid_constant__ State s,
+constexpr int les_ctas() {
+  constexpr int T = FftShape<N>::T;
+  return sizeof(R) == sizeof(double) ? (T <= 64 ? 3 : 1) : (T == 16 || T == 32 ? 5 : 1);
+}
+template <int N, typename R>
+__global__ void __launch_bounds__(3 * FftShape<N>::T * prod_zr<N>(), les_ctas<N, R>()) k_products_les(const __grid_constant__ State s,
                                                                                     Geom g, int zr) {
   using C = typename CplxOf<R>::type;
   using S = FftShape<N>;
